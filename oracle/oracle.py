@@ -52,7 +52,8 @@ _refbk = None
 def build(ref: bool = True) -> None:
     """Compiles the oracle (and, when the reference tree exists, the reference)."""
     targets = ["oracle"]
-    if ref and Path(os.environ.get("DP_REFERENCE", "/root/reference")).exists():
+    tree = Path(os.environ.get("DP_REFERENCE", "/root/reference"))
+    if ref and (tree / "delayed_lu" / "delayed_dgetrf.cpp").exists():
         targets += ["ref", "refgpu", "refbk"]
     env = dict(os.environ)
     if "DP_REFERENCE" in os.environ:
