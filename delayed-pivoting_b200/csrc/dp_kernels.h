@@ -135,6 +135,18 @@ inline bool valid_precision(int precision) {
          precision == DP_PRECISION_MIXED_BF16X6;
 }
 
+// Stream-ordered device memory from the library's two pools (pool.cu), freed
+// with cudaFreeAsync: workspaces of one call, and factors that outlive it.
+cudaError_t workspace_alloc(void** out, size_t bytes, cudaStream_t st);
+cudaError_t resident_alloc(void** out, size_t bytes, cudaStream_t st);
+// Gives the current device's unused pool memory back to the driver.
+void memory_trim();
+// The calling thread's pinned block for device-to-host copies, nullptr when
+// `bytes` exceeds it or it cannot be had; its contents belong to the caller
+// until the next copy this thread makes through it.
+constexpr size_t kPinnedStageBytes = 512 * 1024;
+void* pinned_stage(size_t bytes);
+
 // Full-pivot search over a(k:m, k:n); result in state->fallback.
 void launch_search_active(const double* a, long long lda, int m, int n, int k, State* state,
                           Cand* block_cands, int max_blocks, cudaStream_t s);

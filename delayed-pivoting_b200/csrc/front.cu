@@ -223,9 +223,9 @@ int dp_front_factor(int m, int n, int p, double* d_f, int ldf, int* row_index, i
   int* d_src = nullptr;
   int status = dp::kOk;
   if (p > 0 && tmp_doubles > 0) {
-    if (cudaMallocAsync(reinterpret_cast<void**>(&tmp), sizeof(double) * tmp_doubles, st) !=
+    if (dp::workspace_alloc(reinterpret_cast<void**>(&tmp), sizeof(double) * tmp_doubles, st) !=
             cudaSuccess ||
-        cudaMallocAsync(reinterpret_cast<void**>(&d_src), sizeof(int) * (size_t)p, st) !=
+        dp::workspace_alloc(reinterpret_cast<void**>(&d_src), sizeof(int) * (size_t)p, st) !=
             cudaSuccess) {
       cudaGetLastError();
       status = dp::kAllocationFailed;

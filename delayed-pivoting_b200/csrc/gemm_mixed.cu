@@ -498,7 +498,7 @@ extern "C" int dp_schur_update_mixed_device(int M, int N, int K, const double* A
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t bytes = mixed_scratch_bytes(M, N, K, terms) + 256;
   char* scratch = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), bytes, st) != cudaSuccess) {
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&scratch), bytes, st) != cudaSuccess) {
     cudaGetLastError();
     return kAllocationFailed;
   }

@@ -163,6 +163,9 @@ struct InvPlan {
   long long copy1_cols = 0, copy2_cols = 0;
 };
 
+// The trailing stream's error word follows the state block.
+constexpr size_t kAuxAt = (sizeof(State) + 15) / 16 * 16;
+
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Lays the workspace out from `base` (nullptr: only computes the size).
@@ -177,7 +180,8 @@ size_t layout_workspace(Workspace& ws, char* base, int pivots, int max_ctas, int
   };
   ws.max_ctas = max_ctas;
   ws.w_max = w_max;
-  ws.state = reinterpret_cast<State*>(take(sizeof(State)));
+  ws.state = reinterpret_cast<State*>(take(kAuxAt + sizeof(int)));
+  ws.aux_status = base ? reinterpret_cast<int*>(base + kAuxAt) : nullptr;
   ws.d_ipiv = reinterpret_cast<int*>(take(sizeof(int) * (size_t)std::max(pivots, 1)));
   ws.d_jpiv = reinterpret_cast<int*>(take(sizeof(int) * (size_t)std::max(pivots, 1)));
   ws.slots = reinterpret_cast<unsigned long long*>(
@@ -191,7 +195,6 @@ size_t layout_workspace(Workspace& ws, char* base, int pivots, int max_ctas, int
   if (defer_cap > 0) {
     ws.defer_blk = reinterpret_cast<int*>(take(sizeof(int) * 2 * (size_t)defer_cap));
     ws.defer_ext = reinterpret_cast<int*>(take(sizeof(int) * 4 * (size_t)defer_cap));
-    ws.aux_status = reinterpret_cast<int*>(take(sizeof(int)));
   }
   ws.scratch = base ? base + off : nullptr;
   ws.mixed = mixed_bytes ? reinterpret_cast<void*>(take(mixed_bytes)) : nullptr;
@@ -304,12 +307,39 @@ thread_local HostTrace* g_trace = nullptr;
 
 int read_state(State& hs, const Workspace& ws, cudaStream_t st) {
   const auto t = std::chrono::steady_clock::now();
-  DP_CHECK_CUDA(cudaMemcpyAsync(&hs, ws.state, sizeof(State), cudaMemcpyDeviceToHost, st));
+  State* const stage = static_cast<State*>(pinned_stage(sizeof(State)));
+  DP_CHECK_CUDA(cudaMemcpyAsync(stage ? stage : &hs, ws.state, sizeof(State),
+                                cudaMemcpyDeviceToHost, st));
   DP_CHECK_CUDA(cudaStreamSynchronize(st));
+  if (stage) hs = *stage;
   if (g_trace && g_trace->on) {
     g_trace->wait_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - t).count();
     g_trace->waits += 1;
   }
+  return kOk;
+}
+
+// The results of a factorisation on `st`: its final state, its records and the
+// trailing stream's error word (kOk where there is none).  They lie one after
+// the other at the workspace's start, so one copy brings them all.
+int read_results(State& fin, int* ipiv, int* jpiv, int pivots, int& aux, const Workspace& ws,
+                 cudaStream_t st) {
+  const char* const first = reinterpret_cast<const char*>(ws.state);
+  const size_t at_i = (size_t)(reinterpret_cast<const char*>(ws.d_ipiv) - first);
+  const size_t at_j = (size_t)(reinterpret_cast<const char*>(ws.d_jpiv) - first);
+  const size_t len = sizeof(int) * (size_t)pivots;
+  std::vector<char> pageable;
+  char* stage = static_cast<char*>(pinned_stage(at_j + len));
+  if (!stage) {
+    pageable.resize(at_j + len);
+    stage = pageable.data();
+  }
+  DP_CHECK_CUDA(cudaMemcpyAsync(stage, first, at_j + len, cudaMemcpyDeviceToHost, st));
+  DP_CHECK_CUDA(cudaStreamSynchronize(st));
+  std::memcpy(&fin, stage, sizeof(State));
+  std::memcpy(&aux, stage + kAuxAt, sizeof(int));
+  std::memcpy(ipiv, stage + at_i, len);
+  std::memcpy(jpiv, stage + at_j, len);
   return kOk;
 }
 
@@ -934,7 +964,7 @@ int getrf_device(int m, int n, double* d_a, int lda, int* ipiv, int* jpiv, int* 
   const size_t bytes = layout_workspace(ws, nullptr, pivots, di.sms, w_max, mixed_bytes,
                                         defer_cap, mixed1_bytes, ip);
   char* base = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&base), bytes, st) != cudaSuccess) {
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&base), bytes, st) != cudaSuccess) {
     cudaGetLastError();
     *info = -1;
     return kAllocationFailed;
@@ -985,20 +1015,9 @@ int getrf_device(int m, int n, double* d_a, int lda, int* ipiv, int* jpiv, int* 
     cudaStreamWaitEvent(st, lanes->join, 0);
     cudaEventRecord(lanes->join, lanes->left);
     cudaStreamWaitEvent(st, lanes->join, 0);
-    if (status == kOk &&
-        cudaMemcpyAsync(&aux, ws.aux_status, sizeof(int), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess)
-      status = kCudaFailure;
   }
   State fin{};
-  if (status == kOk) {
-    if (cudaMemcpyAsync(ipiv, ws.d_ipiv, sizeof(int) * pivots, cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(jpiv, ws.d_jpiv, sizeof(int) * pivots, cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(&fin, ws.state, sizeof(State), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-      status = kCudaFailure;
-  }
+  if (status == kOk) status = read_results(fin, ipiv, jpiv, pivots, aux, ws, st);
   cudaFreeAsync(base, st);
   if (cudaStreamSynchronize(st) != cudaSuccess && status == kOk) status = kCudaFailure;
   if (status == kOk && aux != kOk) status = aux;
@@ -1036,7 +1055,7 @@ int getrf_host(int m, int n, double* a, int lda, int* ipiv, int* jpiv, int* info
   size_t bytes = 0;
   if (!matrix_byte_count(lda, n, bytes)) return kInvalidArgument;
   double* d_a = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&d_a), bytes, st) != cudaSuccess) {
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&d_a), bytes, st) != cudaSuccess) {
     cudaGetLastError();
     return kAllocationFailed;
   }
@@ -1064,7 +1083,7 @@ int getrf_host(int m, int n, double* a, int lda, int* ipiv, int* jpiv, int* info
 // CUDA runtime's.  getrf_device_noalloc runs the same plain-FP64 delayed LU
 // as getrf_device but takes its scratch (state block, device swap records,
 // panel swap lists, fallback-search candidates) from one file-scope device
-// array instead of cudaMallocAsync.  It always uses the cluster panel, which
+// array instead of a memory pool.  It always uses the cluster panel, which
 // needs no cross-CTA mailboxes, so the scratch stays small.
 //
 // The array belongs to the library: every GPU that loads it holds
@@ -1151,14 +1170,8 @@ int getrf_device_noalloc(int m, int n, double* d_a, int lda, int* ipiv, int* jpi
   sc.r3 = &rec;
   if (status == kOk) status = factorize(m, n, d_a, lda, o, ws, di, sc, inf);
   State fin{};
-  if (status == kOk) {
-    if (cudaMemcpyAsync(ipiv, ws.d_ipiv, sizeof(int) * pivots, cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(jpiv, ws.d_jpiv, sizeof(int) * pivots, cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(&fin, ws.state, sizeof(State), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-      status = kCudaFailure;
-  }
+  int aux = kOk;
+  if (status == kOk) status = read_results(fin, ipiv, jpiv, pivots, aux, ws, st);
   if (cudaStreamSynchronize(st) != cudaSuccess && status == kOk) status = kCudaFailure;
   if (status != kOk) {
     cudaGetLastError();
@@ -1237,8 +1250,8 @@ int dp_getrf_autotune(int n, int* nb, int* nb_outer, void* stream) {
                                  {128, 128}, {32, 256}, {64, 256}, {128, 256}};
   const size_t elems = (size_t)n * n;
   double *src = nullptr, *work = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&src), sizeof(double) * elems, st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&work), sizeof(double) * elems, st) !=
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&src), sizeof(double) * elems, st) != cudaSuccess ||
+      dp::workspace_alloc(reinterpret_cast<void**>(&work), sizeof(double) * elems, st) !=
           cudaSuccess) {
     cudaGetLastError();
     if (src) cudaFreeAsync(src, st);

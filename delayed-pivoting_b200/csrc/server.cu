@@ -19,7 +19,7 @@
 //   resident   a factorisation with follow-up solves stays on the device
 //              until its last follow-up is done; a stalled refinement on
 //              mixed factors re-factors in FP64 and the factors stay FP64
-// All device memory comes from the stream-ordered pool (cudaMallocAsync), so
+// All device memory comes from the library's stream-ordered pools, so
 // no allocation or release synchronises the device under concurrent work.
 #include <algorithm>
 #include <chrono>
@@ -250,7 +250,7 @@ void dp_server::solve_large(std::vector<Job>& batch, size_t first, Factor* f, co
     const Job& j = batch[first];
     status = dp::factor_solve(f, A, lda, j.r.d_b, j.r.ldb, j.r.nrhs, opt.max_iter, opt.tol, &ir, st);
   } else {
-    if (cudaMallocAsync(reinterpret_cast<void**>(&W), sizeof(double) * (size_t)n * k, st) !=
+    if (dp::workspace_alloc(reinterpret_cast<void**>(&W), sizeof(double) * (size_t)n * k, st) !=
         cudaSuccess) {
       cudaGetLastError();
       W = nullptr;
@@ -412,7 +412,7 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
   auto fail = [&](int status) {
     for (int i = 0; i < k; ++i) out[i].status = status;
   };
-  if (cudaMallocAsync(reinterpret_cast<void**>(&mem), bytes, st) != cudaSuccess) {
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&mem), bytes, st) != cudaSuccess) {
     cudaGetLastError();
     return fail(DP_ALLOCATION_FAILED);
   }
@@ -544,7 +544,7 @@ void dp_server::run_small_new(std::vector<Job>& jobs, cudaStream_t st) {
     r.info = -1;
   }
   int status = DP_SUCCESS;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&g->mem), total, st) != cudaSuccess) {
+  if (dp::resident_alloc(reinterpret_cast<void**>(&g->mem), total, st) != cudaSuccess) {
     cudaGetLastError();
     g->mem = nullptr;
     status = DP_ALLOCATION_FAILED;
@@ -856,6 +856,7 @@ void dp_server_destroy(dp_server* s) {
   cudaStreamSynchronize(st);
   cudaStreamDestroy(st);
   delete s;
+  dp::memory_trim();
 }
 
 }  // extern "C"

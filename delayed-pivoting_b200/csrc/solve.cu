@@ -201,7 +201,7 @@ int lu_solve_inplace(const double* lu, long long ldlu, int n, const double* inv,
 // Flags + status word for lu_solve_inplace at order n (zeroed).
 int alloc_flags(int n, unsigned** flags, cudaStream_t st) {
   const size_t bytes = sizeof(unsigned) * ((size_t)tri_solve_flag_count(n) + 1);
-  if (cudaMallocAsync(reinterpret_cast<void**>(flags), bytes, st) != cudaSuccess) {
+  if (dp::resident_alloc(reinterpret_cast<void**>(flags), bytes, st) != cudaSuccess) {
     cudaGetLastError();
     *flags = nullptr;
     return kAllocationFailed;
@@ -239,20 +239,20 @@ int getrs_device(int n, int nrhs, const double* lu, int ldlu, const int* ipiv, c
   unsigned epoch = 0;
   double* inv = nullptr;
   if (alloc_flags(n, &flags, st) != kOk) return kAllocationFailed;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&inv), sizeof(double) * tri_inverse_doubles(n),
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&inv), sizeof(double) * tri_inverse_doubles(n),
                       st) != cudaSuccess) {
     cudaGetLastError();
     cudaFreeAsync(flags, st);
     return kAllocationFailed;
   }
-  if (cudaMallocAsync(reinterpret_cast<void**>(&d_perm), sizeof(int) * 2 * (size_t)n, st) !=
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&d_perm), sizeof(int) * 2 * (size_t)n, st) !=
       cudaSuccess) {
     cudaGetLastError();
     cudaFreeAsync(flags, st);
     cudaFreeAsync(inv, st);
     return kAllocationFailed;
   }
-  if (cudaMallocAsync(reinterpret_cast<void**>(&tmp), sizeof(double) * (size_t)n * nrhs, st) !=
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&tmp), sizeof(double) * (size_t)n * nrhs, st) !=
       cudaSuccess) {
     cudaGetLastError();
     cudaFreeAsync(d_perm, st);
@@ -419,11 +419,11 @@ int factor_condest(Factor* f, const double* A, int lda, double* kappa, double* i
     cudaStreamSynchronize(st);
   };
   const size_t nb = (size_t)(n + 63) / 64;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&lut), sizeof(double) * (size_t)n * n, st) !=
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&lut), sizeof(double) * (size_t)n * n, st) !=
           cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&inv_t), sizeof(double) * tri_inverse_doubles(n),
+      dp::workspace_alloc(reinterpret_cast<void**>(&inv_t), sizeof(double) * tri_inverse_doubles(n),
                       st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&vec), sizeof(double) * 4 * (size_t)n, st) !=
+      dp::workspace_alloc(reinterpret_cast<void**>(&vec), sizeof(double) * 4 * (size_t)n, st) !=
           cudaSuccess) {
     cudaGetLastError();
     release();
@@ -547,11 +547,11 @@ int factor_create(Factor** out, int n, const double* A, int lda, int precision, 
   f->ipiv.resize(n);
   f->jpiv.resize(n);
   double* normA = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void**>(&f->lu), sizeof(double) * (size_t)n * n, st) !=
+  if (dp::resident_alloc(reinterpret_cast<void**>(&f->lu), sizeof(double) * (size_t)n * n, st) !=
           cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&f->d_perm), sizeof(int) * 2 * (size_t)n, st) !=
+      dp::resident_alloc(reinterpret_cast<void**>(&f->d_perm), sizeof(int) * 2 * (size_t)n, st) !=
           cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&normA), sizeof(double), st) != cudaSuccess) {
+      dp::workspace_alloc(reinterpret_cast<void**>(&normA), sizeof(double), st) != cudaSuccess) {
     cudaGetLastError();
     if (normA) cudaFreeAsync(normA, st);
     factor_destroy(f, st);
@@ -559,7 +559,7 @@ int factor_create(Factor** out, int n, const double* A, int lda, int precision, 
   }
   int status = alloc_flags(n, &f->d_flags, st);
   if (status == kOk &&
-      cudaMallocAsync(reinterpret_cast<void**>(&f->d_inv), sizeof(double) * tri_inverse_doubles(n),
+      dp::resident_alloc(reinterpret_cast<void**>(&f->d_inv), sizeof(double) * tri_inverse_doubles(n),
                       st) != cudaSuccess) {
     cudaGetLastError();
     f->d_inv = nullptr;
@@ -589,7 +589,7 @@ int factor_create(Factor** out, int n, const double* A, int lda, int precision, 
     double range[2] = {0.0, INFINITY};
     double* scr = nullptr;
     if (status == kOk &&
-        cudaMallocAsync(reinterpret_cast<void**>(&scr), 2 * sizeof(double), st) != cudaSuccess) {
+        dp::workspace_alloc(reinterpret_cast<void**>(&scr), 2 * sizeof(double), st) != cudaSuccess) {
       cudaGetLastError();
       status = kAllocationFailed;
     }
@@ -657,10 +657,10 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
     if (norms) cudaFreeAsync(norms, st);
     cudaStreamSynchronize(st);
   };
-  if (cudaMallocAsync(reinterpret_cast<void**>(&X), nr * sizeof(double), st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&R), nr * sizeof(double), st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&T), nr * sizeof(double), st) != cudaSuccess ||
-      cudaMallocAsync(reinterpret_cast<void**>(&norms), 2 * (size_t)nrhs * sizeof(double), st) !=
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&X), nr * sizeof(double), st) != cudaSuccess ||
+      dp::workspace_alloc(reinterpret_cast<void**>(&R), nr * sizeof(double), st) != cudaSuccess ||
+      dp::workspace_alloc(reinterpret_cast<void**>(&T), nr * sizeof(double), st) != cudaSuccess ||
+      dp::workspace_alloc(reinterpret_cast<void**>(&norms), 2 * (size_t)nrhs * sizeof(double), st) !=
           cudaSuccess) {
     cudaGetLastError();
     release();

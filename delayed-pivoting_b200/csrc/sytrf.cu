@@ -707,7 +707,7 @@ int sytrf_device(int n, double* d_a, int lda, int* perm, int* piv_size, int* inf
   const size_t b_int = align256((size_t)n * sizeof(int));
   const size_t total = b_wt + 2 * b_vec + b_cp + b_rp + 2 * b_int + align256(sizeof(bk::State));
   char* ws = nullptr;
-  if (cudaMallocAsync((void**)&ws, total, s) != cudaSuccess) return kAllocationFailed;
+  if (workspace_alloc((void**)&ws, total, s) != cudaSuccess) return kAllocationFailed;
   bk::State hs;  // the panel kernel's state, read after each launch (a few bytes)
   bk::State* h = &hs;
   bk::Params P;
@@ -748,13 +748,16 @@ int sytrf_device(int n, double* d_a, int lda, int* perm, int* piv_size, int* inf
     rec.begin(DP_KFAM_PANEL);
     const long long per_slot = (long long)G * bk::kRowsPerCta;
     const int slots = (int)((n - pb + per_slot - 1) / per_slot);
+    void* const stage = pinned_stage(sizeof(bk::State));
     if (cudaLaunchCooperativeKernel(bk::panel_kernel_for(slots), dim3(G), dim3(bk::kThreads), args,
                                     0, s) != cudaSuccess ||
-        cudaMemcpyAsync(h, P.st, sizeof(bk::State), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaMemcpyAsync(stage ? stage : h, P.st, sizeof(bk::State), cudaMemcpyDeviceToHost, s) !=
+            cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
       status = kCudaFailure;
       break;
     }
+    if (stage) std::memcpy(h, stage, sizeof(bk::State));
     {
       // algorithmic traffic of the launch: per factored column the column and
       // row reads and the L and W column writes over the rows below pb

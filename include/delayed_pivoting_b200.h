@@ -351,6 +351,10 @@ int dp_server_poll(dp_server *server, dp_request_result *out, int max, int wait_
 int dp_server_stats_get(dp_server *server, dp_server_stats *out);
 /* Seconds on the server's monotonic clock (the timestamps of the results). */
 double dp_server_clock(void);
+
+/* Device memory that calls have freed is kept for the next one (at most 4 GiB
+ * a device); this gives the current device's back to the driver. */
+int dp_memory_trim(void);
 /* Waits for every queued request, releases all resident factors, stops. */
 void dp_server_destroy(dp_server *server);
 
