@@ -166,24 +166,19 @@ void launch_set_record(int* ipiv, int* jpiv, int k, int p, int q, cudaStream_t s
 
 // ---- triangular solves with many right-hand sides (trisolve.cu) ----------
 
-// Y (n x nrhs, nrhs <= tri_solve_rhs_max()) <- L^{-1} Y (unit lower) or
-// U^{-1} Y (upper with diagonal), one launch; `flags` holds
-// tri_solve_flag_count(n) words: one per 64-row block, whose values differ
-// from `epoch` (nonzero, new for every launch that uses the same flags), then
-// the launch's block-ticket counter (reset by the launch); a bounded wait
-// that runs out sets *status = kDeviceTimeout.
-// `inv` holds the inverses of the 64 x 64 diagonal blocks of L and U
-// (launch_diag_inverse, tri_inverse_doubles(n) doubles, 16-byte aligned).
-int tri_solve_rhs_max();
-int tri_solve_flag_count(int n);
+// X <- Q U^{-1} L^{-1} P B (n x nrhs) in one launch per 64 right-hand sides:
+// row / col are the composite orders (B row row[i] is eliminated i-th, unknown
+// col[i] takes the i-th value), X may be B.  `inv` holds the inverses of the
+// 64 x 64 diagonal blocks of L and U (launch_diag_inverse,
+// tri_inverse_doubles(n) doubles, 16-byte aligned), `work`
+// lu_solve_work_bytes(n, nrhs) bytes; a bounded wait that runs out sets
+// *status = kDeviceTimeout.
 size_t tri_inverse_doubles(int n);
 int launch_diag_inverse(const double* lu, long long ldlu, int n, double* inv, cudaStream_t st);
-int launch_tri_lower_unit(const double* L, long long ldl, int n, const double* inv, double* Y,
-                          long long ldy, int nrhs, unsigned* flags, unsigned epoch, int* status,
-                          cudaStream_t st);
-int launch_tri_upper(const double* U, long long ldu, int n, const double* inv, double* Y,
-                     long long ldy, int nrhs, unsigned* flags, unsigned epoch, int* status,
-                     cudaStream_t st);
+size_t lu_solve_work_bytes(int n, int nrhs);
+int launch_lu_solve(const double* lu, long long ldlu, int n, const double* inv, const int* row,
+                    const int* col, const double* B, long long ldb, double* X, long long ldx,
+                    int nrhs, void* work, int* status, cudaStream_t st);
 
 // ---- resident factorisations (solve.cu) ----------------------------------
 
@@ -198,9 +193,7 @@ struct Factor {
   double factor_ms = 0.0;             // device time of all factorisations
   double* lu = nullptr;
   int* d_perm = nullptr;              // row order [n], column order [n]
-  unsigned* d_flags = nullptr;        // triangular-solve block flags, then a status word
   double* d_inv = nullptr;            // inverses of the diagonal blocks of L and U
-  unsigned epoch = 0;                 // last epoch used on d_flags
   int panel_rows = 0;                 // rows per panel CTA of its factorisations (0: default)
   std::vector<int> ipiv, jpiv;
 };

@@ -81,7 +81,12 @@ struct Job {
   std::shared_ptr<Resident> res;     // follow-ups
 };
 
-size_t scratch_bytes(int n, int nrhs) {  // X, R, T of one solve, its columns in a coalesced solve
+// X, R and the two buffers of one solve, its columns in a coalesced solve.
+size_t scratch_bytes(int n, int nrhs) { return 5 * sizeof(double) * (size_t)n * nrhs + 4096; }
+
+// The smallest scratch a budget must hold beside the factor for a request to
+// be accepted; one between the two is charged all that the budget has left.
+size_t least_scratch_bytes(int n, int nrhs) {
   return 4 * sizeof(double) * (size_t)n * nrhs + 4096;
 }
 
@@ -787,7 +792,8 @@ int dp_server_submit(dp_server* s, const dp_request* q) {
   j.scratch = scratch_bytes(r.n, r.nrhs);
   if (r.factor_id == 0)
     j.factor = s->is_small(r.n) ? small_factor_bytes(r.n) : large_factor_bytes(r.n);
-  if (j.scratch + j.factor > s->budget) return DP_INVALID_ARGUMENT;
+  if (least_scratch_bytes(r.n, r.nrhs) + j.factor > s->budget) return DP_INVALID_ARGUMENT;
+  j.scratch = std::min(j.scratch, s->budget - j.factor);
   std::lock_guard<std::mutex> lk(s->m);
   if (s->stop) return DP_INVALID_ARGUMENT;
   if (r.factor_id == 0) {

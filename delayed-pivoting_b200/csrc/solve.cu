@@ -31,26 +31,6 @@ int getrf_device(int m, int n, double* d_a, int lda, int* ipiv, int* jpiv, int* 
 
 namespace {
 
-__global__ void gather_rows_kernel(const double* __restrict__ in, long long ldi, double* out,
-                                   long long ldo, const int* __restrict__ perm, int n, int nrhs) {
-  const long long total = (long long)n * nrhs;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n), c = (int)(e / n);
-    out[idx(i, c, ldo)] = in[idx(perm[i], c, ldi)];
-  }
-}
-
-__global__ void scatter_rows_kernel(const double* __restrict__ in, long long ldi, double* out,
-                                    long long ldo, const int* __restrict__ perm, int n, int nrhs) {
-  const long long total = (long long)n * nrhs;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n), c = (int)(e / n);
-    out[idx(perm[i], c, ldo)] = in[idx(i, c, ldi)];
-  }
-}
-
 __global__ void copy_kernel(const double* __restrict__ in, long long ldi, double* out, long long ldo,
                             int n, int nrhs) {
   const long long total = (long long)n * nrhs;
@@ -101,28 +81,33 @@ __global__ void diag_range_kernel(const double* __restrict__ D, long long ldd, i
   }
 }
 
-// out[c] = max_i |X(i, c)| (out must be zero on entry); NaN is reported as +inf.
-__global__ void colmax_kernel(const double* __restrict__ X, long long ldx, int n, int nrhs,
-                              double* out) {
-  const int c = blockIdx.y;
-  double m = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double v = fabs(X[idx(i, c, ldx)]);
-    m = (v == v) ? fmax(m, v) : __longlong_as_double(0x7ff0000000000000ll);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, off));
-  if ((threadIdx.x & 31) == 0) atomic_max_pos(out + c, m);
-}
-
-// rowsum[i] = sum_j |A(i, j)| over the n x n matrix (threads over rows, so
-// each column is read coalesced); out[0] = max_i rowsum (atomic).
-__global__ void row_abs_sum_kernel(const double* __restrict__ A, long long lda, int n, double* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// out[0] = max_i sum_j |A(i, j)| over the n x n matrix (zero on entry; NaN
+// reported as +inf).  32 rows a CTA, a lane a row, warp w the columns w, w +
+// 8, .. with 16 loads in flight: with a thread per row the device was nearly
+// empty (n = 10000: 1.0 ms, 0.8 TB/s).
+__global__ void __launch_bounds__(256) row_abs_sum_kernel(const double* __restrict__ A,
+                                                          long long lda, int n, double* out) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  const double* const a = A + min(row, n - 1);
   double s = 0.0;
-  if (i < n)
-    for (int j = 0; j < n; ++j) s += fabs(A[idx(i, j, lda)]);
-  if (i < n) atomic_max_pos(out, s == s ? s : __longlong_as_double(0x7ff0000000000000ll));
+  for (int j0 = warp; j0 < n; j0 += 128) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = j0 + 8 * u < n ? a[(long long)(j0 + 8 * u) * lda] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) s += fabs(v[u]);
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) s += part[w][lane];
+  s = row >= n ? 0.0 : s == s ? s : __longlong_as_double(0x7ff0000000000000ll);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) s = fmax(s, __shfl_down_sync(0xffffffffu, s, off));
+  if (lane == 0) atomic_max_pos(out, s);
 }
 
 // out (n x n, leading dimension n) = in^T.  32 x 32 tiles through shared
@@ -177,50 +162,6 @@ int grid_of(long long work) {
 
 }  // namespace
 
-// T (n x nrhs at leading dimension n) <- U^{-1} L^{-1} T with the compact L\U
-// at lu: the two triangular solves in launches of up to tri_solve_rhs_max()
-// right-hand sides, each with a fresh epoch of `flags`.
-int lu_solve_inplace(const double* lu, long long ldlu, int n, const double* inv, double* T,
-                     int nrhs, unsigned* flags, unsigned& epoch, cudaStream_t st) {
-  int* status = reinterpret_cast<int*>(flags + tri_solve_flag_count(n));
-  const int cmax = tri_solve_rhs_max();
-  for (int c0 = 0; c0 < nrhs; c0 += cmax) {
-    const int nc = std::min(cmax, nrhs - c0);
-    for (int up = 0; up < 2; ++up) {
-      if (++epoch == 0) ++epoch;
-      const int s = up ? launch_tri_upper(lu, ldlu, n, inv, T + (size_t)c0 * n, n, nc, flags,
-                                          epoch, status, st)
-                       : launch_tri_lower_unit(lu, ldlu, n, inv, T + (size_t)c0 * n, n, nc,
-                                               flags, epoch, status, st);
-      if (s != kOk) return s;
-    }
-  }
-  return kOk;
-}
-
-// Flags + status word for lu_solve_inplace at order n (zeroed).
-int alloc_flags(int n, unsigned** flags, cudaStream_t st) {
-  const size_t bytes = sizeof(unsigned) * ((size_t)tri_solve_flag_count(n) + 1);
-  if (dp::resident_alloc(reinterpret_cast<void**>(flags), bytes, st) != cudaSuccess) {
-    cudaGetLastError();
-    *flags = nullptr;
-    return kAllocationFailed;
-  }
-  if (cudaMemsetAsync(*flags, 0, bytes, st) != cudaSuccess) return kCudaFailure;
-  return kOk;
-}
-
-// kOk, or the status a triangular solve left in the flags' status word
-// (synchronises st).
-int solve_status(const unsigned* flags, int n, cudaStream_t st) {
-  int h = 0;
-  if (cudaMemcpyAsync(&h, flags + tri_solve_flag_count(n), sizeof(int), cudaMemcpyDeviceToHost,
-                      st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return kCudaFailure;
-  return h == 0 ? kOk : h;
-}
-
 int getrs_device(int n, int nrhs, const double* lu, int ldlu, const int* ipiv, const int* jpiv,
                  double* B, int ldb, cudaStream_t st) {
   if (n < 0 || nrhs < 0 || ldlu < std::max(1, n) || ldb < std::max(1, n)) return kInvalidArgument;
@@ -233,84 +174,170 @@ int getrs_device(int n, int nrhs, const double* lu, int ldlu, const int* ipiv, c
     std::swap(row[k], row[ipiv[k]]);
     std::swap(col[k], col[jpiv[k]]);
   }
-  int* d_perm = nullptr;
-  double* tmp = nullptr;
-  unsigned* flags = nullptr;
-  unsigned epoch = 0;
-  double* inv = nullptr;
-  if (alloc_flags(n, &flags, st) != kOk) return kAllocationFailed;
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&inv), sizeof(double) * tri_inverse_doubles(n),
-                      st) != cudaSuccess) {
+  // status word, then the composite orders, the diagonal inverses, the solve's buffers
+  const size_t b_perm = sizeof(int) * (4 + 2 * (((size_t)n + 1) & ~(size_t)1));
+  const size_t b_inv = sizeof(double) * tri_inverse_doubles(n);
+  char* mem = nullptr;
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&mem),
+                          b_perm + b_inv + lu_solve_work_bytes(n, nrhs), st) != cudaSuccess) {
     cudaGetLastError();
-    cudaFreeAsync(flags, st);
     return kAllocationFailed;
   }
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&d_perm), sizeof(int) * 2 * (size_t)n, st) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    cudaFreeAsync(flags, st);
-    cudaFreeAsync(inv, st);
-    return kAllocationFailed;
-  }
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&tmp), sizeof(double) * (size_t)n * nrhs, st) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    cudaFreeAsync(d_perm, st);
-    cudaFreeAsync(flags, st);
-    cudaFreeAsync(inv, st);
-    return kAllocationFailed;
-  }
-  int status = kOk;
-  if (cudaMemcpyAsync(d_perm, row.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st) !=
+  int* const d_status = reinterpret_cast<int*>(mem);
+  int* const d_perm = d_status + 4;
+  double* const inv = reinterpret_cast<double*>(mem + b_perm);
+  int status = kOk, h = kOk;
+  if (cudaMemsetAsync(d_status, 0, sizeof(int), st) != cudaSuccess ||
+      cudaMemcpyAsync(d_perm, row.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st) !=
           cudaSuccess ||
       cudaMemcpyAsync(d_perm + n, col.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st) !=
           cudaSuccess)
     status = kCudaFailure;
-  if (status == kOk) {
-    const long long total = (long long)n * nrhs;
-    dp::note_launch();
-    gather_rows_kernel<<<grid_of(total), 256, 0, st>>>(B, ldb, tmp, n, d_perm, n, nrhs);
-    status = launch_diag_inverse(lu, ldlu, n, inv, st);
-    if (status == kOk) status = lu_solve_inplace(lu, ldlu, n, inv, tmp, nrhs, flags, epoch, st);
-    if (status == kOk) {
-      dp::note_launch();
-      scatter_rows_kernel<<<grid_of(total), 256, 0, st>>>(tmp, n, B, ldb, d_perm + n, n, nrhs);
-    }
-    if (cudaGetLastError() != cudaSuccess && status == kOk) status = kCudaFailure;
-    if (status == kOk) status = solve_status(flags, n, st);
-  }
-  cudaFreeAsync(tmp, st);
-  cudaFreeAsync(d_perm, st);
-  cudaFreeAsync(flags, st);
-  cudaFreeAsync(inv, st);
+  if (status == kOk) status = launch_diag_inverse(lu, ldlu, n, inv, st);
+  if (status == kOk)
+    status = launch_lu_solve(lu, ldlu, n, inv, d_perm, d_perm + n, B, ldb, B, ldb, nrhs,
+                             mem + b_perm + b_inv, d_status, st);
+  if (status == kOk &&
+      cudaMemcpyAsync(&h, d_status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    status = kCudaFailure;
+  cudaFreeAsync(mem, st);
   if (cudaStreamSynchronize(st) != cudaSuccess && status == kOk) status = kCudaFailure;
-  return status;
+  return status == kOk ? h : status;
 }
 
 namespace {
 
-// max over columns of ||R_c|| / (normA ||X_c|| + ||B_c||), all infinity norms.
+__device__ __forceinline__ double finite_or_inf(double v) {  // NaN counts as +inf
+  return v == v ? fabs(v) : __longlong_as_double(0x7ff0000000000000ll);
+}
+
+// R = B - A X and, per column c, the largest |R|, |X| and |B| in norms[c],
+// norms[nrhs + c], norms[2 nrhs + c] (zero on entry).
+// Bound: A is read once per group of NC right-hand sides, by 32 rows a CTA so
+// that n = 4096 already fills the device; a lane owns a row, warp w the
+// columns 32 (8 s + w) .. of A, with 16 loads of A in flight per lane while
+// the previous 16 are multiplied (the right-hand sides come from shared
+// memory, a broadcast).  The eight partial sums of a row are added in warp
+// order, so the result does not depend on the launch.  With the update kernel
+// in its place (64-row tiles, 64 CTAs at n = 4096, a copy and two norm
+// launches beside it) the residual took 150 us with one right-hand side,
+// against 21 us for reading A.
+constexpr int kResT = 256, kResW = kResT / 32, kResK = 16;
+
+template <int NC>
+__global__ void __launch_bounds__(kResT, NC <= 8 ? 2 : 1)
+residual_kernel(const double* __restrict__ A, long long lda, int n, const double* __restrict__ B,
+                long long ldb, const double* __restrict__ X, long long ldx, int nrhs, double* R,
+                long long ldr, double* norms) {
+  extern __shared__ __align__(16) double rsm[];  // [kResW][32][NC]: X, then the partial sums
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r0 = blockIdx.y * 32, row = r0 + lane, c0 = blockIdx.x * NC;
+  const int nc = min(NC, nrhs - c0);
+  const double* const arow = A + min(row, n - 1);
+  double* const xw = rsm + warp * 32 * NC;
+  double acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+  double a[2][kResK];
+  auto load = [&](double (&t)[kResK], int k0) {
+#pragma unroll
+    for (int k = 0; k < kResK; ++k) t[k] = k0 + k < n ? arow[(long long)(k0 + k) * lda] : 0.0;
+  };
+  int k0 = warp * 32;
+  if (k0 < n) load(a[0], k0);
+  for (; k0 < n; k0 += 32 * kResW) {
+    __syncwarp();  // xw is free
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+      xw[lane * NC + c] = (c < nc && k0 + lane < n) ? X[(k0 + lane) + (long long)(c0 + c) * ldx] : 0.0;
+    load(a[1], k0 + kResK);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < kResK; ++k)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = fma(a[0][k], xw[k * NC + c], acc[c]);
+    if (k0 + 32 * kResW < n) load(a[0], k0 + 32 * kResW);
+#pragma unroll
+    for (int k = 0; k < kResK; ++k)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = fma(a[1][k], xw[(kResK + k) * NC + c], acc[c]);
+  }
+  __syncthreads();  // every warp is done with X
+#pragma unroll
+  for (int c = 0; c < NC; ++c) rsm[(warp * NC + c) * 32 + lane] = acc[c];
+  __syncthreads();
+  for (int c = warp; c < nc; c += kResW) {
+    double s = 0.0, m[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int w = 0; w < kResW; ++w) s += rsm[(w * NC + c) * 32 + lane];
+    if (row < n) {
+      const double b = B[row + (long long)(c0 + c) * ldb];
+      const double r = b - s;
+      R[row + (long long)(c0 + c) * ldr] = r;
+      m[0] = finite_or_inf(r);
+      m[1] = finite_or_inf(X[row + (long long)(c0 + c) * ldx]);
+      m[2] = finite_or_inf(b);
+    }
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) m[t] = fmax(m[t], __shfl_down_sync(~0u, m[t], off));
+      if (lane == 0) atomic_max_pos(norms + (size_t)t * nrhs + c0 + c, m[t]);
+    }
+  }
+}
+
+template <int NC>
+int launch_residual(const double* A, int lda, int n, const double* B, int ldb, const double* X,
+                    int ldx, int nrhs, double* R, double* norms, cudaStream_t st) {
+  const size_t smem = sizeof(double) * kResW * 32 * NC;
+  if (!ensure_smem((const void*)residual_kernel<NC>, smem)) return kCudaFailure;
+  dp::note_launch();
+  residual_kernel<NC><<<dim3((nrhs + NC - 1) / NC, (n + 31) / 32), kResT, smem, st>>>(
+      A, lda, n, B, ldb, X, ldx, nrhs, R, n, norms);
+  return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
+}
+
+// R = B - A X and berr = max over columns of ||R_c|| / (normA ||X_c|| +
+// ||B_c||), all infinity norms.  `head` (device, solve_head_bytes(nrhs)):
+// the solve's status word, then the norms; a timed-out solve is reported.
+size_t solve_head_bytes(int nrhs) { return 16 + sizeof(double) * 3 * (size_t)nrhs; }
+
 int backward_error(const double* A, int lda, int n, const double* B, int ldb, const double* X,
-                   int ldx, int nrhs, double* R, double* norms, double normA,
-                   const std::vector<double>& normB, double& berr, cudaStream_t st) {
-  const long long total = (long long)n * nrhs;
-  dp::note_launch();
-  copy_kernel<<<grid_of(total), 256, 0, st>>>(B, ldb, R, n, n, nrhs);
-  launch_gemm_minus(n, nrhs, n, A, lda, X, ldx, R, n, st);
-  if (cudaMemsetAsync(norms, 0, sizeof(double) * 2 * nrhs, st) != cudaSuccess) return kCudaFailure;
-  dim3 g((unsigned)std::min(64, (n + 255) / 256), (unsigned)nrhs);
-  dp::note_launch();
-  colmax_kernel<<<g, 256, 0, st>>>(R, n, n, nrhs, norms);
-  dp::note_launch();
-  colmax_kernel<<<g, 256, 0, st>>>(X, ldx, n, nrhs, norms + nrhs);
-  std::vector<double> h(2 * (size_t)nrhs);
-  if (cudaMemcpyAsync(h.data(), norms, sizeof(double) * 2 * nrhs, cudaMemcpyDeviceToHost, st) !=
+                   int ldx, int nrhs, double* R, char* head, double normA, double& berr,
+                   cudaStream_t st) {
+  double* const norms = reinterpret_cast<double*>(head + 16);
+  if (cudaMemsetAsync(norms, 0, sizeof(double) * 3 * nrhs, st) != cudaSuccess) return kCudaFailure;
+  // as many right-hand sides a CTA as there are (A is read once per group), but
+  // no more than eight while the CTAs would not fill the device: n = 2311 with
+  // 32 has 73 row blocks
+  const int blocks = (n + 31) / 32, sms = sm_count();
+  int nc = nrhs <= 1 ? 1 : nrhs <= 4 ? 4 : nrhs <= 8 ? 8 : nrhs <= 16 ? 16 : 32;
+  while (nc > 8 && (long long)blocks * ((nrhs + nc - 1) / nc) < sms) nc /= 2;
+  auto launch = nc == 1    ? launch_residual<1>
+                : nc == 4  ? launch_residual<4>
+                : nc == 8  ? launch_residual<8>
+                : nc == 16 ? launch_residual<16>
+                           : launch_residual<32>;
+  if (int rc = launch(A, lda, n, B, ldb, X, ldx, nrhs, R, norms, st)) return rc;
+  std::vector<double> own;
+  const size_t bytes = solve_head_bytes(nrhs);
+  const double* h = static_cast<const double*>(pinned_stage(bytes));
+  if (!h) {
+    own.resize(bytes / sizeof(double));
+    h = own.data();
+  }
+  if (cudaMemcpyAsync(const_cast<double*>(h), head, bytes, cudaMemcpyDeviceToHost, st) !=
           cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return kCudaFailure;
+  int solve = kOk;
+  std::memcpy(&solve, h, sizeof(int));
+  if (solve != kOk) return solve;
+  h += 2;
   berr = 0.0;
   for (int c = 0; c < nrhs; ++c) {
-    const double den = normA * h[nrhs + c] + normB[c];
+    const double den = normA * h[nrhs + c] + h[2 * nrhs + c];
     const double e = den > 0.0 ? h[c] / den : (h[c] > 0.0 ? INFINITY : 0.0);
     berr = std::max(berr, std::isnan(e) ? INFINITY : e);
   }
@@ -359,40 +386,22 @@ int factorize(Factor& f, const double* A, int lda, int prec, cudaStream_t st) {
   return kOk;
 }
 
-// X = A^{-1} B through the factors (X, tmp: n x nrhs, leading dimension n).
-int solve_with(Factor& f, const double* B, int ldb, double* X, double* tmp, int nrhs,
-               cudaStream_t st) {
-  const int n = f.n;
-  const long long total = (long long)n * nrhs;
-  dp::note_launch();
-  gather_rows_kernel<<<grid_of(total), 256, 0, st>>>(B, ldb, tmp, n, f.d_perm, n, nrhs);
-  const int s = lu_solve_inplace(f.lu, n, n, f.d_inv, tmp, nrhs, f.d_flags, f.epoch, st);
-  if (s != kOk) return s;
-  dp::note_launch();
-  scatter_rows_kernel<<<grid_of(total), 256, 0, st>>>(tmp, n, X, n, f.d_perm + n, n, nrhs);
-  return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
+// X = A^{-1} B through the factors (X: n x nrhs, leading dimension n; it may
+// be B); `work` as for launch_lu_solve.
+int solve_with(const Factor& f, const double* B, int ldb, double* X, void* work, int nrhs,
+               int* status, cudaStream_t st) {
+  return launch_lu_solve(f.lu, f.n, f.n, f.d_inv, f.d_perm, f.d_perm + f.n, B, ldb, X, f.n, nrhs,
+                         work, status, st);
 }
 
 // z = A^{-T} c through the factors: A^T = Q U^T L^T P, so with w[k] =
 // c[col[k]]: U^T v = w (lower solve on the transposed factor T = (L\U)^T),
 // L^T u = v (upper solve on T), z[row[k]] = u[k].  `lut` / `inv_t` are the
 // transpose of the compact factor and its transposed diagonal inverses.
-int solve_transposed(Factor& f, const double* lut, const double* inv_t, const double* c, double* z,
-                     double* tmp, cudaStream_t st) {
-  const int n = f.n;
-  dp::note_launch();
-  gather_rows_kernel<<<grid_of(n), 256, 0, st>>>(c, n, tmp, n, f.d_perm + n, n, 1);
-  int* status = reinterpret_cast<int*>(f.d_flags + tri_solve_flag_count(n));
-  for (int up = 0; up < 2; ++up) {
-    if (++f.epoch == 0) ++f.epoch;
-    const int s = up ? launch_tri_upper(lut, n, n, inv_t, tmp, n, 1, f.d_flags, f.epoch, status, st)
-                     : launch_tri_lower_unit(lut, n, n, inv_t, tmp, n, 1, f.d_flags, f.epoch,
-                                             status, st);
-    if (s != kOk) return s;
-  }
-  dp::note_launch();
-  scatter_rows_kernel<<<grid_of(n), 256, 0, st>>>(tmp, n, z, n, f.d_perm, n, 1);
-  return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
+int solve_transposed(const Factor& f, const double* lut, const double* inv_t, const double* c,
+                     double* z, void* work, int* status, cudaStream_t st) {
+  return launch_lu_solve(lut, f.n, f.n, inv_t, f.d_perm + f.n, f.d_perm, c, f.n, z, f.n, 1, work,
+                         status, st);
 }
 
 }  // namespace
@@ -423,22 +432,26 @@ int factor_condest(Factor* f, const double* A, int lda, double* kappa, double* i
           cudaSuccess ||
       dp::workspace_alloc(reinterpret_cast<void**>(&inv_t), sizeof(double) * tri_inverse_doubles(n),
                       st) != cudaSuccess ||
-      dp::workspace_alloc(reinterpret_cast<void**>(&vec), sizeof(double) * 4 * (size_t)n, st) !=
-          cudaSuccess) {
+      dp::workspace_alloc(reinterpret_cast<void**>(&vec), sizeof(double) * (5 * (size_t)n + 4),
+                          st) != cudaSuccess) {
     cudaGetLastError();
     release();
     return kAllocationFailed;
   }
   double* x = vec;          // input of a solve
   double* y = vec + n;      // its result
-  double* tmp = vec + 2 * (size_t)n;
-  double* colsum = vec + 3 * (size_t)n;
+  double* colsum = vec + 2 * (size_t)n;
+  void* work = vec + 3 * (size_t)n;
+  int* d_status = reinterpret_cast<int*>(vec + 5 * (size_t)n + 2);
   dp::note_launch(3);
   transpose_kernel<<<dim3((n + 31) / 32, (n + 31) / 32), dim3(32, 8), 0, st>>>(f->lu, n, lut, n);
   transpose_inverses_kernel<<<grid_of((long long)(2 * 64 * 64 * nb)), 256, 0, st>>>(f->d_inv, inv_t,
                                                                                   (int)nb);
   col_abs_sum_kernel<<<(int)(((long long)n * 32 + 255) / 256), 256, 0, st>>>(A, lda, n, colsum);
-  int status = cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
+  int status = cudaGetLastError() == cudaSuccess &&
+                       cudaMemsetAsync(d_status, 0, sizeof(int), st) == cudaSuccess
+                   ? kOk
+                   : kCudaFailure;
   std::vector<double> hx(n), hy(n), hsum(n);
   auto down = [&](std::vector<double>& h, const double* d) {
     if (status == kOk && (cudaMemcpyAsync(h.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost,
@@ -452,11 +465,11 @@ int factor_condest(Factor* f, const double* A, int lda, double* kappa, double* i
       status = kCudaFailure;
   };
   auto forward = [&] {  // y = A^{-1} x (x on the device), copied to hy
-    if (status == kOk) status = solve_with(*f, x, n, y, tmp, 1, st);
+    if (status == kOk) status = solve_with(*f, x, n, y, work, 1, d_status, st);
     down(hy, y);
   };
   auto backward = [&] {  // y = A^{-T} x, copied to hy
-    if (status == kOk) status = solve_transposed(*f, lut, inv_t, x, y, tmp, st);
+    if (status == kOk) status = solve_transposed(*f, lut, inv_t, x, y, work, d_status, st);
     down(hy, y);
   };
   down(hsum, colsum);
@@ -510,7 +523,12 @@ int factor_condest(Factor* f, const double* A, int lda, double* kappa, double* i
     for (double v : hy) s1 += std::fabs(v);
     est = std::max(est, 2.0 * s1 / (3.0 * n));
   }
-  if (status == kOk && f->d_flags) status = solve_status(f->d_flags, n, st);
+  int timed_out = kOk;
+  if (status == kOk && (cudaMemcpyAsync(&timed_out, d_status, sizeof(int), cudaMemcpyDeviceToHost,
+                                        st) != cudaSuccess ||
+                        cudaStreamSynchronize(st) != cudaSuccess))
+    status = kCudaFailure;
+  if (status == kOk) status = timed_out;
   release();
   if (status != kOk) return status;
   if (inv_norm) *inv_norm = est;
@@ -522,15 +540,13 @@ void factor_destroy(Factor* f, cudaStream_t st) {
   if (!f) return;
   if (f->lu) cudaFreeAsync(f->lu, st);
   if (f->d_perm) cudaFreeAsync(f->d_perm, st);
-  if (f->d_flags) cudaFreeAsync(f->d_flags, st);
   if (f->d_inv) cudaFreeAsync(f->d_inv, st);
   cudaStreamSynchronize(st);
   delete f;
 }
 
 size_t factor_bytes(int n) {
-  return sizeof(double) * ((size_t)n * n + tri_inverse_doubles(n)) + sizeof(int) * 2 * (size_t)n +
-         sizeof(unsigned) * ((size_t)tri_solve_flag_count(n) + 1);
+  return sizeof(double) * ((size_t)n * n + tri_inverse_doubles(n)) + sizeof(int) * 2 * (size_t)n;
 }
 
 int factor_create(Factor** out, int n, const double* A, int lda, int precision, cudaStream_t st,
@@ -557,9 +573,8 @@ int factor_create(Factor** out, int n, const double* A, int lda, int precision, 
     factor_destroy(f, st);
     return kAllocationFailed;
   }
-  int status = alloc_flags(n, &f->d_flags, st);
-  if (status == kOk &&
-      dp::resident_alloc(reinterpret_cast<void**>(&f->d_inv), sizeof(double) * tri_inverse_doubles(n),
+  int status = kOk;
+  if (dp::resident_alloc(reinterpret_cast<void**>(&f->d_inv), sizeof(double) * tri_inverse_doubles(n),
                       st) != cudaSuccess) {
     cudaGetLastError();
     f->d_inv = nullptr;
@@ -573,7 +588,7 @@ int factor_create(Factor** out, int n, const double* A, int lda, int precision, 
   if (cudaMemsetAsync(normA, 0, sizeof(double), st) != cudaSuccess) status = kCudaFailure;
   if (status == kOk) {
     dp::note_launch();
-    row_abs_sum_kernel<<<(n + 255) / 256, 256, 0, st>>>(A, lda, n, normA);
+    row_abs_sum_kernel<<<(n + 31) / 32, 256, 0, st>>>(A, lda, n, normA);
     if (cudaMemcpyAsync(&f->normA, normA, sizeof(double), cudaMemcpyDeviceToHost, st) !=
             cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
@@ -649,43 +664,27 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
     return kOk;
   }
   const size_t nr = (size_t)n * nrhs;
-  double *X = nullptr, *R = nullptr, *T = nullptr, *norms = nullptr;
-  auto release = [&] {
-    if (X) cudaFreeAsync(X, st);
-    if (R) cudaFreeAsync(R, st);
-    if (T) cudaFreeAsync(T, st);
-    if (norms) cudaFreeAsync(norms, st);
-    cudaStreamSynchronize(st);
-  };
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&X), nr * sizeof(double), st) != cudaSuccess ||
-      dp::workspace_alloc(reinterpret_cast<void**>(&R), nr * sizeof(double), st) != cudaSuccess ||
-      dp::workspace_alloc(reinterpret_cast<void**>(&T), nr * sizeof(double), st) != cudaSuccess ||
-      dp::workspace_alloc(reinterpret_cast<void**>(&norms), 2 * (size_t)nrhs * sizeof(double), st) !=
-          cudaSuccess) {
+  // one block: status word and norms, X, R, the solve's buffers
+  const size_t b_head = (solve_head_bytes(nrhs) + 255) / 256 * 256;
+  const size_t b_vec = (nr * sizeof(double) + 255) / 256 * 256;
+  char* head = nullptr;
+  if (dp::workspace_alloc(reinterpret_cast<void**>(&head),
+                          b_head + 2 * b_vec + lu_solve_work_bytes(n, nrhs), st) != cudaSuccess) {
     cudaGetLastError();
-    release();
     return kAllocationFailed;
   }
-  std::vector<double> normB(nrhs);
-  int status = kOk;
-  {
-    if (cudaMemsetAsync(norms, 0, sizeof(double) * nrhs, st) != cudaSuccess) status = kCudaFailure;
-    dim3 g((unsigned)std::min(64, (n + 255) / 256), (unsigned)nrhs);
-    dp::note_launch();
-    colmax_kernel<<<g, 256, 0, st>>>(B, ldb, n, nrhs, norms);
-    if (status == kOk &&
-        (cudaMemcpyAsync(normB.data(), norms, sizeof(double) * nrhs, cudaMemcpyDeviceToHost, st) !=
-             cudaSuccess ||
-         cudaStreamSynchronize(st) != cudaSuccess))
-      status = kCudaFailure;
-  }
+  double* const X = reinterpret_cast<double*>(head + b_head);
+  double* const R = reinterpret_cast<double*>(head + b_head + b_vec);
+  void* const work = head + b_head + 2 * b_vec;
+  int* const d_status = reinterpret_cast<int*>(head);
+  int status = cudaMemsetAsync(head, 0, sizeof(int), st) == cudaSuccess ? kOk : kCudaFailure;
 
   auto refine = [&](int iters_left, bool& converged) -> int {
     converged = false;
     double prev = INFINITY;
     for (int it = 0;; ++it) {
       double berr = INFINITY;
-      int s = backward_error(A, lda, n, B, ldb, X, n, nrhs, R, norms, f->normA, normB, berr, st);
+      int s = backward_error(A, lda, n, B, ldb, X, n, nrhs, R, head, f->normA, berr, st);
       if (s != kOk) return s;
       res->backward_error = berr;
       if (berr <= tol) {
@@ -702,7 +701,7 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
         if (it + needed > iters_left + 0.5) return kOk;
       }
       prev = berr;
-      s = solve_with(*f, R, n, R, T, nrhs, st);
+      s = solve_with(*f, R, n, R, work, nrhs, d_status, st);
       if (s != kOk) return s;
       dp::note_launch();
       axpy_kernel<<<grid_of((long long)nr), 256, 0, st>>>(R, n, X, n, n, nrhs);
@@ -717,7 +716,7 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
   const double fms0 = f->factor_ms - res->factor_ms;
   bool converged = false;
   if (status == kOk) {
-    status = solve_with(*f, B, ldb, X, T, nrhs, st);
+    status = solve_with(*f, B, ldb, X, work, nrhs, d_status, st);
     if (status == kOk) status = refine(max_iter, converged);
   }
   if (status == kOk && !converged && f->precision != DP_PRECISION_FP64) {
@@ -725,18 +724,11 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
     f->refactored = 1;
     status = factorize(*f, A, lda, DP_PRECISION_FP64, st);
     if (status == kOk && f->info == n) {
-      status = solve_with(*f, B, ldb, X, T, nrhs, st);
+      status = solve_with(*f, B, ldb, X, work, nrhs, d_status, st);
       if (status == kOk) status = refine(max_iter, converged);
     }
   }
   cudaEventRecord(t1, st);
-  cudaEventSynchronize(t1);
-  float tot = 0.f;
-  cudaEventElapsedTime(&tot, t0, t1);
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
-  if (status == kOk) status = solve_status(f->d_flags, n, st);
-  res->total_ms = tot;
   res->factor_ms = f->factor_ms - fms0;
   res->info = f->info;
   res->refactored = f->refactored;
@@ -745,7 +737,13 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
     dp::note_launch();
     copy_kernel<<<grid_of((long long)nr), 256, 0, st>>>(X, n, B, ldb, n, nrhs);
   }
-  release();
+  cudaFreeAsync(head, st);
+  if (cudaStreamSynchronize(st) != cudaSuccess && status == kOk) status = kCudaFailure;
+  float tot = 0.f;
+  cudaEventElapsedTime(&tot, t0, t1);
+  cudaEventDestroy(t0);
+  cudaEventDestroy(t1);
+  res->total_ms = tot;
   return status;
 }
 

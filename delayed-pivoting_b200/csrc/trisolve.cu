@@ -1,26 +1,36 @@
-// Triangular solves with many right-hand sides in ONE launch (the solve and
-// refinement path: getrs and every refinement correction).
+// X = Q U^{-1} L^{-1} P B with many right-hand sides in ONE launch: the solve of
+// getrs and of every refinement step, the row order of the factorisation
+// applied while B is read and its column order while X is written.
 //
-// Y (n x nrhs, nrhs <= 64) <- T^{-1} Y with T the unit-lower L or the upper U
-// (with its diagonal) of a compact L\U factorisation.  The rows are cut into
-// blocks of 64; a grid of up to one CTA per SM takes the blocks in dependency order
-// (lower: top down, upper: bottom up) by tickets from an atomic counter, so
-// every block a CTA waits for was claimed earlier by a CTA that is already
-// running: the earliest unfinished block always has every input it needs,
-// and no CTA depends on one that has not started - no co-residency (no
-// cooperative launch) is needed, and the launch starts on whatever SMs are
-// free.  A block
-//   1. starts from its rows of Y,
-//   2. for each earlier block j: waits until j is published (a flag set to the
-//      launch's epoch, read with acquire semantics, bounded by kSpinLimitNs),
-//      stages y_j in shared memory and subtracts T(i, j) y_j; T(i, j) arrives
-//      by asynchronous copies issued one block ahead (T read once),
-//   3. multiplies by the inverse of its 64 x 64 diagonal block (inverses made
-//      once per factorisation by diag_inverse_kernel, staged in shared memory
-//      while the dependencies were awaited) - a product over all threads
-//      instead of a 64-step serial substitution on the critical path,
-//   4. writes y_i and publishes it (fence, then a release store of the flag).
-// A wait that runs out sets *status = kDeviceTimeout and every CTA returns.
+// Work is cut into tasks (row block of 64, group of NC right-hand sides): the
+// L tasks top down, then the U tasks bottom up, each level over all groups.
+// CTAs take tasks by tickets from an atomic counter, so every block a task
+// waits for was claimed earlier by a CTA that is already running: no
+// co-residency (no cooperative launch) is needed, and the launch starts on
+// whatever SMs are free.  A task
+//   1. starts from its rows of P B (L) or of L's result (U),
+//   2. for each earlier block j: waits for that block's values, puts them in
+//      shared memory and subtracts T(i, j) y_j, T(i, j) held in registers and
+//      loaded one block ahead (each T element is read once per group);
+//      thread (r, q) takes row r and the 16 columns 16 q .. of every block.
+//      The four partial sums of a block are folded into the row's value
+//      behind the next block's barrier: kept apart until the end they lose
+//      the cancellation that keeps an elimination's intermediate values
+//      small, and the solutions were 1.2 - 1.7 times further off,
+//   3. multiplies by the inverse of its 64 x 64 diagonal block (made once per
+//      factorisation by diag_inverse_kernel, staged in shared memory while the
+//      dependencies were awaited) - a product over all threads instead of a
+//      64-step serial substitution,
+//   4. publishes its values.
+// The values are their own flag: the result buffers start as all-ones bit
+// patterns (a NaN that no task publishes: a result with that pattern is
+// written as the ordinary NaN), and a consumer polls the element it needs.
+// The chain of blocks bounds the launch (2 n / 64 links): with a separate flag
+// per block - a fence, a release store, an acquire poll and then a second
+// round trip to L2 for the values - and one CTA for all right-hand sides a
+// link took 2.9 us with one right-hand side (n = 4096: 186 us a triangle) and
+// 13 us with 32 (n = 2311: 490 us).
+// A wait that runs out sets *status = kDeviceTimeout; every CTA then returns.
 #include <algorithm>
 #include <atomic>
 
@@ -30,47 +40,34 @@
 namespace dp {
 namespace {
 
-constexpr int kTB = 64;           // rows per block
-constexpr int kTT = 256;          // threads
-constexpr int kTRhs = 64;         // right-hand sides per launch
-constexpr int kTAcc = kTRhs / 4;  // accumulators per thread (4 column groups)
-constexpr int kTMaxGrid = 32;     // CTAs of one launch under a block-count policy
+constexpr int kTB = 64;        // rows per block
+constexpr int kTT = 256;       // threads
+constexpr int kTQ = kTT / kTB; // column quarters of a block
+constexpr int kTK = kTB / kTQ; // columns per quarter
+constexpr int kTRhs = 64;      // right-hand sides per launch
+constexpr int kTMaxGrid = 32;  // CTAs of one launch under a block-count policy
 
-// CTAs of a launch (dp_tri_solve_grid): 0 -> min(blocks, SMs); g > 0 ->
-// min(blocks, g); g < 0 -> one CTA per -g row blocks (at most kTMaxGrid).
+constexpr unsigned long long kUnset = ~0ull;  // not yet published
+
+// CTAs of a launch (dp_tri_solve_grid): 0 -> as many as fit; g > 0 -> at most
+// g; g < 0 -> one CTA per -g row blocks (at most kTMaxGrid).
 std::atomic<int> g_tri_grid{0};
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned long long ld_relaxed(const double* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void publish(double* p, double v) {
+  unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  if (u == kUnset) u = 0x7ff8000000000000ull;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
 }
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// T(r0 + k, c0 + c) for k, c < 64 into sm[c * kTB + k] (zeros outside the
-// rows x cols block), 8-byte asynchronous copies.
-__device__ __forceinline__ void stage_block(double* sm, const double* T, long long ldt, int r0,
-                                            int c0, int rows, int cols) {
-  for (int e = threadIdx.x; e < kTB * kTB; e += kTT) {
-    const int k = e & (kTB - 1), c = e >> 6;
-    if (k < rows && c < cols)
-      cp_async8(sm + e, T + (r0 + k) + (long long)(c0 + c) * ldt);
-    else
-      sm[e] = 0.0;
-  }
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
 // inv + 2 * kTB * kTB * i holds, column-major, the inverse of the unit-lower
@@ -139,204 +136,221 @@ __global__ void __launch_bounds__(kTT) diag_inverse_kernel(const double* __restr
   }
 }
 
-__device__ __forceinline__ void cp_async16(double* dst, const double* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+struct SolveParams {
+  const double* lu;
+  long long ldlu;
+  int n;
+  const double* inv;
+  const int *row, *col;  // composite row / column orders
+  const double* B;
+  long long ldb;
+  double* X;
+  long long ldx;
+  int nrhs;
+  double* mid;   // n x nrhs, L's result; all ones on entry
+  double* xs;    // n x nrhs, U's result in elimination order; all ones on entry
+  int* counter;  // all ones on entry
+  int* status;
+};
+
+template <int NC>
+constexpr size_t solve_smem() {
+  return sizeof(double) * (2 * kTB * NC + 2 * kTQ * kTB * NC + kTB * kTB);
 }
 
-// MACC accumulators per thread: columns cg, cg + 4, ..., cg + 4 (MACC - 1)
-// (nrhs <= 4 MACC), so a launch with few right-hand sides issues no idle FMAs.
-template <bool kUpper, int MACC>
-__global__ void __launch_bounds__(kTT, 1) tri_solve_kernel(const double* __restrict__ T,
-                                                           long long ldt, int n,
-                                                           const double* __restrict__ inv,
-                                                           double* Y, long long ldy, int nrhs,
-                                                           unsigned* flags, unsigned epoch,
-                                                           int* status) {
-  constexpr int kNp = MACC == 1 ? 4 : 1;  // partial sums per accumulator
-  extern __shared__ double tsm[];
-  double* ys = tsm;                  // y_j, [kTRhs][kTB]
-  double* ds = ys + kTB * kTRhs;     // the block's right-hand sides, [kTRhs][kTB]
-  double* dg = ds + kTB * kTRhs;     // diagonal block T(i, i), [kTB][kTB] column-major
-  double* ls = dg + kTB * kTB;       // T(i, j) double buffer, 2 x [kTB][kTB]
-  __shared__ int abort_all, ticket;
-  const int tid = threadIdx.x, r = tid & (kTB - 1), cg = tid >> 6;
-  const int nblk = (n + kTB - 1) / kTB;
-  int* const counter = reinterpret_cast<int*>(flags + nblk);  // zeroed before the launch
-  if (tid == 0) abort_all = 0;
+// The values of rows [r0, r0 + rows) and columns [c0, c0 + nc) of `src` once
+// they are published, as dst[k * NC + c] (zeros elsewhere); false when the
+// wait runs out or another CTA's did.
+template <int NC>
+__device__ __forceinline__ bool await_values(double* dst, const double* src, int n, int r0, int rows,
+                                             int c0, int nc, const int* status) {
+  constexpr int kPer = (kTB * NC + kTT - 1) / kTT;
+  unsigned long long v[kPer];
+  bool want[kPer], all;
+  unsigned long long t0 = 0;
+  for (unsigned it = 0;; ++it) {
+    all = true;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int e = (int)threadIdx.x + u * kTT, k = e & (kTB - 1), c = e >> 6;
+      want[u] = c < nc && k < rows;
+      v[u] = want[u] ? ld_relaxed(src + (r0 + k) + (long long)(c0 + c) * n) : 0ull;
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) all = all && v[u] != kUnset;
+    if (all) break;
+    if ((it & 63u) == 63u) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kSpinLimitNs || ld_volatile_i32(status) != kOk) break;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int e = (int)threadIdx.x + u * kTT, k = e & (kTB - 1), c = e >> 6;
+    if (c < NC) dst[k * NC + c] = __longlong_as_double((long long)v[u]);
+  }
+  return all;
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kTT, 2) lu_solve_kernel(const __grid_constant__ SolveParams p) {
+  extern __shared__ __align__(16) double tsm[];
+  double* const ys = tsm;                      // [2][kTB][NC] values of the block in hand
+  double* const red = ys + 2 * kTB * NC;       // [2][kTQ][NC][kTB] partial sums
+  double* const dg = red + 2 * kTQ * kTB * NC; // inverse of the diagonal block, column-major
+  constexpr int kOwn = (NC + kTQ - 1) / kTQ;   // columns q, q + kTQ, .. of row r: this thread's
+  __shared__ int ticket;
+  const int tid = threadIdx.x, r = tid & (kTB - 1), q = tid >> 6;
+  const int n = p.n, nblk = (n + kTB - 1) / kTB;
+  const int groups = (p.nrhs + NC - 1) / NC;
+  const int tasks = 2 * nblk * groups;
   for (;;) {
-    if (tid == 0) ticket = atomicAdd(counter, 1);
+    __syncthreads();  // ticket, ys, red and dg are free
+    if (tid == 0) ticket = atomicAdd(p.counter, 1) + 1;
     __syncthreads();
-    const int q = ticket;
-    __syncthreads();  // every thread holds q before the next claim
-    if (q >= nblk || abort_all) break;
-    const int i = kUpper ? nblk - 1 - q : q;
+    const int task = ticket;
+    if (task >= tasks) return;
+    const int level = task / groups, c0 = (task - level * groups) * NC;
+    const int nc = min(NC, p.nrhs - c0);
+    const bool up = level >= nblk;
+    const int i = up ? 2 * nblk - 1 - level : level;
     const int r0 = i * kTB, rows = min(kTB, n - r0);
-    const int deps = kUpper ? nblk - 1 - i : i;
-    // the diagonal block and the first off-diagonal block, in flight while
-    // the dependencies are awaited
+    const int deps = up ? nblk - 1 - i : i;
     {
-      const double* src = inv + (size_t)2 * kTB * kTB * i + (kUpper ? kTB * kTB : 0);
+      const double* src = p.inv + (size_t)2 * kTB * kTB * i + (up ? kTB * kTB : 0);
       for (int e = 2 * tid; e < kTB * kTB; e += 2 * kTT) cp_async16(dg + e, src + e);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    cp_async_commit();
-    auto dep = [&](int t) { return kUpper ? nblk - 1 - t : t; };
-    if (deps > 0) {
-      const int j = dep(0);
-      stage_block(ls, T, ldt, r0, j * kTB, rows, min(kTB, n - j * kTB));
-    }
-    cp_async_commit();
-    double acc[MACC];
+    // T(i, j)'s part of this thread: row r, columns 16 q + k
+    const double* const trow = p.lu + (r0 + r) + (long long)(kTK * q) * p.ldlu;
+    auto load_tile = [&](double (&t)[kTK], int d) {
+      const int j = up ? nblk - 1 - d : d;
+      const double* src = trow + (long long)j * kTB * p.ldlu;
+      const int left = n - j * kTB - kTK * q;  // columns of this quarter inside the matrix
 #pragma unroll
-    for (int m = 0; m < MACC; ++m) {
-      const int c = cg + 4 * m;
-      acc[m] = (r < rows && c < nrhs) ? Y[(r0 + r) + c * ldy] : 0.0;
-    }
-    // thread 0 confirms block dep(t) before the barrier that opens step t
-    auto await_dep = [&](int t) {
-      if (tid != 0 || abort_all) return;
-      const int j = dep(t);
-      const unsigned long long t0 = globaltimer_ns();
-      while (ld_acquire_u32(flags + j) != epoch) {
-        if (globaltimer_ns() - t0 > kSpinLimitNs) {
-          abort_all = 1;
-          atomicExch(status, kDeviceTimeout);
-          break;
-        }
-      }
+      for (int k = 0; k < kTK; ++k)
+        t[k] = (r < rows && k < left) ? src[(long long)k * p.ldlu] : 0.0;
     };
-    if (deps > 0) await_dep(0);
-    __syncthreads();
-    for (int t = 0; t < deps; ++t) {
-      if (abort_all) {
-        cp_async_wait<0>();
-        return;
+    double tile[2][kTK];
+    if (deps > 0) load_tile(tile[0], 0);
+    double acc[NC], own[kOwn];
+#pragma unroll
+    for (int u = 0; u < kOwn; ++u) own[u] = 0.0;
+    bool good = true;
+    if (up) {
+      // L's result at this block: awaited like any other block's values
+      good = await_values<NC>(ys, p.mid, n, r0, rows, c0, nc, p.status);
+      if (!__syncthreads_and(good)) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (tid == 0) atomicCAS(p.status, kOk, kDeviceTimeout);
+        break;
       }
-      const int j = dep(t);
-      const int rj = j * kTB, rowsj = min(kTB, n - rj);
-      double* lb = ls + (t & 1) * kTB * kTB;
-      if (t + 1 < deps) {  // the next block's T(i, j') behind this one
-        const int jn = dep(t + 1);
-        stage_block(ls + ((t + 1) & 1) * kTB * kTB, T, ldt, r0, jn * kTB, rows,
-                    min(kTB, n - jn * kTB));
-      }
-      cp_async_commit();
-      for (int e = tid; e < kTB * nrhs; e += kTT) {
-        const int k = e & (kTB - 1), c = e >> 6;
-        ys[e] = k < rowsj ? __ldcg(Y + (rj + k) + c * ldy) : 0.0;
-      }
-      cp_async_wait<1>();  // lb has landed (the newest group may still be in flight)
+#pragma unroll
+      for (int u = 0; u < kOwn; ++u)
+        if (q + u * kTQ < NC) own[u] = ys[r * NC + q + u * kTQ];
       __syncthreads();
-      if (r < rows) {
-        // kNp interleaved partial sums (few right-hand sides: the per-thread
-        // FMA chain, not the issue rate, bounds this step)
-        double part[kNp][MACC];  // part[0] unused: the first sum is acc
+    } else if (r < rows && q < nc) {
+      const long long src = p.row[r0 + r];
 #pragma unroll
-        for (int q = 0; q < kNp; ++q)
-#pragma unroll
-          for (int m = 0; m < MACC; ++m) part[q][m] = 0.0;
-#pragma unroll 8
-        for (int k = 0; k < kTB; k += kNp) {
-#pragma unroll
-          for (int q = 0; q < kNp; ++q) {
-            const double l = lb[(k + q) * kTB + r];
-#pragma unroll
-            for (int m = 0; m < MACC; ++m)
-              if (cg + 4 * m < nrhs) {
-                double& dst = q == 0 ? acc[m] : part[q][m];
-                dst = fma(-l, ys[(cg + 4 * m) * kTB + k + q], dst);
-              }
-          }
-        }
-#pragma unroll
-        for (int m = 0; m < MACC; ++m)
-#pragma unroll
-          for (int q = 1; q < kNp; ++q) acc[m] += part[q][m];
-      }
-      if (t + 1 < deps) await_dep(t + 1);
-      __syncthreads();  // ys and lb are free; the next dependency is confirmed
+      for (int u = 0; u < kOwn; ++u)
+        if (q + u * kTQ < nc) own[u] = p.B[src + (long long)(c0 + q + u * kTQ) * p.ldb];
     }
-    cp_async_wait<0>();
+    // the four partial sums of block d, in the order of its columns
+    auto folded = [&](int d, int c) {
+      const double* s = red + ((d & 1) * kTQ * NC + c) * kTB + r;
+      return (s[0] + s[NC * kTB]) + (s[2 * NC * kTB] + s[3 * NC * kTB]);
+    };
+    auto put = [&](int d) {
 #pragma unroll
-    for (int m = 0; m < MACC; ++m) {
-      const int c = cg + 4 * m;
-      if (c < nrhs) ds[c * kTB + r] = acc[m];
+      for (int c = 0; c < NC; ++c) red[(((d & 1) * kTQ + q) * NC + c) * kTB + r] = acc[c];
+    };
+    auto fold = [&](int d) {
+#pragma unroll
+      for (int u = 0; u < kOwn; ++u)
+        if (q + u * kTQ < NC) own[u] -= folded(d, q + u * kTQ);
+    };
+    const double* const from = up ? p.xs : p.mid;
+    auto step = [&](const double (&t)[kTK], double (&next)[kTK], int d) -> bool {
+      const int j = up ? nblk - 1 - d : d;
+      if (d + 1 < deps) load_tile(next, d + 1);
+      double* const y = ys + (d & 1) * kTB * NC;
+      good = await_values<NC>(y, from, n, j * kTB, min(kTB, n - j * kTB), c0, nc, p.status);
+      // (this half of ys and of red was last read before the previous barrier)
+      if (!__syncthreads_and(good)) return false;
+      const double* yq = y + kTK * q * NC;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+#pragma unroll
+      for (int k = 0; k < kTK; ++k)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) acc[c] = fma(t[k], yq[k * NC + c], acc[c]);
+      put(d);
+      if (d > 0) fold(d - 1);
+      return true;
+    };
+    bool ok = true;
+    for (int d = 0; ok && d < deps; d += 2) {
+      ok = step(tile[0], tile[1], d);
+      if (ok && d + 1 < deps) ok = step(tile[1], tile[0], d + 1);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!ok) {
+      if (tid == 0) atomicCAS(p.status, kOk, kDeviceTimeout);
+      break;
+    }
+    // the last block's partial sums, then the diagonal block's inverse
     __syncthreads();
-    // y_i = inverse(T(i, i)) * (right-hand sides): thread (r, cg) forms rows
-    // r of its columns
-    if (r < rows) {
-      double y[MACC], yp[kNp][MACC];  // yp[0] unused: the first sum is y
+    if (deps > 0) fold(deps - 1);
+    double* const y = ys + (deps & 1) * kTB * NC;
 #pragma unroll
-      for (int m = 0; m < MACC; ++m) {
-        y[m] = 0.0;
-#pragma unroll
-        for (int q = 0; q < kNp; ++q) yp[q][m] = 0.0;
-      }
-#pragma unroll 8
-      for (int k = 0; k < kTB; k += kNp) {
-#pragma unroll
-        for (int q = 0; q < kNp; ++q) {
-          const double a = dg[(k + q) * kTB + r];
-#pragma unroll
-          for (int m = 0; m < MACC; ++m)
-            if (cg + 4 * m < nrhs) {
-              double& dst = q == 0 ? y[m] : yp[q][m];
-              dst = fma(a, ds[(cg + 4 * m) * kTB + k + q], dst);
-            }
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < MACC; ++m)
-#pragma unroll
-        for (int q = 1; q < kNp; ++q) y[m] += yp[q][m];
-#pragma unroll
-      for (int m = 0; m < MACC; ++m) {
-        const int c = cg + 4 * m;
-        if (c < nrhs) Y[(r0 + r) + c * ldy] = y[m];
-      }
-    }
+    for (int u = 0; u < kOwn; ++u)
+      if (q + u * kTQ < NC) y[r * NC + q + u * kTQ] = own[u];
     __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      st_release_u32(flags + i, epoch);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) acc[c] = 0.0;
+#pragma unroll
+    for (int k = 0; k < kTK; ++k) {
+      const double a = dg[(kTK * q + k) * kTB + r];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) acc[c] = fma(a, y[(kTK * q + k) * NC + c], acc[c]);
     }
+    put(deps);
+    __syncthreads();
+    const long long xrow = up && r < rows ? p.col[r0 + r] : 0;
+#pragma unroll
+    for (int u = 0; u < kOwn; ++u)
+      if (const int c = q + u * kTQ; c < nc && r < rows) {
+        const double s = folded(deps, c);
+        const size_t at = (size_t)(r0 + r) + (size_t)(c0 + c) * n;
+        publish((up ? p.xs : p.mid) + at, s);
+        if (up) p.X[xrow + (long long)(c0 + c) * p.ldx] = s;
+      }
   }
 }
 
-template <bool kUpper, int MACC>
-int launch_tri(const double* T, long long ldt, int n, const double* inv, double* Y,
-               long long ldy, int nrhs, unsigned* flags, unsigned epoch, int* status,
-               cudaStream_t st) {
-  const size_t smem = sizeof(double) * (2 * kTB * kTRhs + 3 * kTB * kTB);
-  if (!ensure_smem((const void*)tri_solve_kernel<kUpper, MACC>, smem)) return kCudaFailure;
+template <int NC>
+int launch_solve(const SolveParams& p, cudaStream_t st) {
+  const void* fn = (const void*)lu_solve_kernel<NC>;
+  const size_t smem = solve_smem<NC>();
+  if (!ensure_smem(fn, smem)) return kCudaFailure;
   const int sms = sm_count();
-  const int per_sm = occupancy_once((const void*)tri_solve_kernel<kUpper, MACC>, kTT, smem);
+  const int per_sm = occupancy_once(fn, kTT, smem);
   if (sms < 1 || per_sm < 1) return kCudaFailure;
-  // Besides the chain of diagonal blocks, block i subtracts all i blocks
-  // before it, T(i, 0:i) y(0:i): that work (the triangle, read once) spreads
-  // over the CTAs, so one CTA per SM is the default - measured against 32
-  // CTAs: n = 16384, one right-hand side, 2.6 ms against 6.1 per solve;
-  // n = 8192 1.06 against 1.80; n = 4096 0.56 against 0.67.
-  const int nblk = (n + kTB - 1) / kTB;
+  const int nblk = (p.n + kTB - 1) / kTB;
+  const int per_level = (p.nrhs + NC - 1) / NC;
   const int policy = g_tri_grid.load(std::memory_order_relaxed);
-  const int want = policy == 0 ? sms
+  const int most = policy == 0 ? sms * per_sm
                    : policy > 0 ? policy
-                                : std::max(1, std::min(kTMaxGrid, (nblk - policy - 1) / -policy));
-  const int grid = std::max(1, std::min(std::min(nblk, want), sms * per_sm));
-  // the ticket counter after the block flags
-  if (cudaMemsetAsync(flags + nblk, 0, sizeof(unsigned), st) != cudaSuccess) return kCudaFailure;
+                                : std::min(kTMaxGrid, (nblk - policy - 1) / -policy);
+  const int grid = std::max(1, std::min({nblk * per_level, most, sms * per_sm}));
   note_launch();
-  tri_solve_kernel<kUpper, MACC><<<grid, kTT, smem, st>>>(T, ldt, n, inv, Y, ldy, nrhs, flags,
-                                                          epoch, status);
-  if (cudaGetLastError() != cudaSuccess) return kCudaFailure;
-  return kOk;
+  lu_solve_kernel<NC><<<grid, kTT, smem, st>>>(p);
+  return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
 }
 
 }  // namespace
 
-int tri_solve_rhs_max() { return kTRhs; }
-int tri_solve_flag_count(int n) { return (n + kTB - 1) / kTB + 1; }  // block flags, ticket
 size_t tri_inverse_doubles(int n) { return (size_t)2 * kTB * kTB * ((n + kTB - 1) / kTB); }
 
 int launch_diag_inverse(const double* lu, long long ldlu, int n, double* inv, cudaStream_t st) {
@@ -346,24 +360,44 @@ int launch_diag_inverse(const double* lu, long long ldlu, int n, double* inv, cu
   return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
 }
 
-int launch_tri_lower_unit(const double* L, long long ldl, int n, const double* inv, double* Y,
-                          long long ldy, int nrhs, unsigned* flags, unsigned epoch, int* status,
-                          cudaStream_t st) {
-  if (n <= 0 || nrhs <= 0) return kOk;
-  if (nrhs > kTRhs) return kInvalidArgument;
-  if (nrhs <= 4) return launch_tri<false, 1>(L, ldl, n, inv, Y, ldy, nrhs, flags, epoch, status, st);
-  if (nrhs <= 16) return launch_tri<false, 4>(L, ldl, n, inv, Y, ldy, nrhs, flags, epoch, status, st);
-  return launch_tri<false, kTAcc>(L, ldl, n, inv, Y, ldy, nrhs, flags, epoch, status, st);
+size_t lu_solve_work_bytes(int n, int nrhs) {
+  return sizeof(double) * 2 * (size_t)n * std::min(nrhs, kTRhs) + 16;
 }
 
-int launch_tri_upper(const double* U, long long ldu, int n, const double* inv, double* Y,
-                     long long ldy, int nrhs, unsigned* flags, unsigned epoch, int* status,
-                     cudaStream_t st) {
+int launch_lu_solve(const double* lu, long long ldlu, int n, const double* inv, const int* row,
+                    const int* col, const double* B, long long ldb, double* X, long long ldx,
+                    int nrhs, void* work, int* status, cudaStream_t st) {
   if (n <= 0 || nrhs <= 0) return kOk;
-  if (nrhs > kTRhs) return kInvalidArgument;
-  if (nrhs <= 4) return launch_tri<true, 1>(U, ldu, n, inv, Y, ldy, nrhs, flags, epoch, status, st);
-  if (nrhs <= 16) return launch_tri<true, 4>(U, ldu, n, inv, Y, ldy, nrhs, flags, epoch, status, st);
-  return launch_tri<true, kTAcc>(U, ldu, n, inv, Y, ldy, nrhs, flags, epoch, status, st);
+  for (int c0 = 0; c0 < nrhs; c0 += kTRhs) {
+    SolveParams p;
+    p.lu = lu;
+    p.ldlu = ldlu;
+    p.n = n;
+    p.inv = inv;
+    p.row = row;
+    p.col = col;
+    p.B = B + (size_t)c0 * ldb;
+    p.ldb = ldb;
+    p.X = X + (size_t)c0 * ldx;
+    p.ldx = ldx;
+    p.nrhs = std::min(kTRhs, nrhs - c0);
+    p.mid = static_cast<double*>(work);
+    p.xs = p.mid + (size_t)n * p.nrhs;
+    p.counter = reinterpret_cast<int*>(p.xs + (size_t)n * p.nrhs);
+    p.status = status;
+    if (cudaMemsetAsync(work, 0xFF, lu_solve_work_bytes(n, p.nrhs), st) != cudaSuccess)
+      return kCudaFailure;
+    // Right-hand sides per task: few columns are computed that are not there,
+    // and at most eight, so that a link of the chain stays short (a block's
+    // product takes 64 NC cycles of the FP64 pipe) and the groups spread over
+    // the SMs.
+    const int rc = p.nrhs == 1   ? launch_solve<1>(p, st)
+                   : p.nrhs == 2 ? launch_solve<2>(p, st)
+                   : p.nrhs <= 4 ? launch_solve<4>(p, st)
+                                 : launch_solve<8>(p, st);
+    if (rc != kOk) return rc;
+  }
+  return kOk;
 }
 
 }  // namespace dp
