@@ -8,12 +8,14 @@
 // histories, compact L\U in place).  Blocking only changes rounding, so the
 // records equal the single-matrix path's and the reference's.
 //
-// One CTA of 256 threads factors one matrix at a time; CTAs pull matrix
-// indices from a device work queue ordered largest first, so the tail is
-// short.  Per panel of nb <= 32 columns:
-//   panel      the n - b panel rows live in REGISTERS, two rows per thread,
-//              thread t owning panel rows t and t + 256 for the whole panel,
-//              factored in sub-panels of 8 columns with a rank-8 update of
+// One CTA factors one matrix at a time; CTAs pull matrix indices from a device
+// work queue ordered largest first, so the tail is short.  The orders fall into
+// four size classes with a CTA shape each (Geo), launched one behind the other
+// so that a class's CTAs take the SMs the class before leaves free
+// (programmatic dependent launch).  Per panel of nb columns (at most the
+// class's window of 16):
+//   panel      the n - b panel rows live in REGISTERS, a row per thread for the
+//              whole panel, factored in sub-panels of 8 columns with a rank-8 update of
 //              the rest of the register window after each.  A row swap only
 //              exchanges the logical positions the owners keep (no data
 //              moves); the candidate for column s + 1 is taken while column
@@ -24,14 +26,11 @@
 //              never wins (delayed_dgetrf_cuda.cu:13-20, :46).
 //   write-back the panel, in logical row order, to the matrix and to shared
 //              memory (L11 and L21 for the update)
-//   permute    the panel's composite row permutation (at most 2 nb rows move)
-//              on every column outside it, four lanes per column gathering
-//              the moved rows into registers before storing them
-//   update     per 256 trailing columns: U12 = L11^{-1} A12 (one thread per
-//              column, in registers) written to the matrix and to a shared
-//              tile, then A22 -= L21 U12 on the FP64 tensor path (mma.sync
-//              m16n8k4, warp tiles 32 x 32, C prefetched into registers
-//              before the k-loop)
+//   update     per STAGE trailing columns: the panel's composite row
+//              permutation (at most 2 nb rows move) and U12 = L11^{-1} A12,
+//              through a shared tile, then A22 -= L21 U12 on the FP64 tensor
+//              path (mma.sync m16n8k4, warp tiles 32 x 32)
+//   left       the permutations owed to the finished columns, once per matrix
 //   fallback   materialize the far columns with the executed prefix, 2-D
 //              argmax (smaller column, then smaller row on ties), full-row and
 //              full-column swaps, restart the panel at k with the pivot placed
@@ -56,21 +55,27 @@
 namespace dp {
 namespace batch {
 
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
-constexpr int kRpt = 2;                   // panel rows per thread
-constexpr int kMaxN = kThreads * kRpt;    // 512
-constexpr int kMaxNb = 32;                // panel width limit = register window
+constexpr int kMaxN = DP_BATCH_MAX_N;
+constexpr int kMaxNb = DP_BATCH_MAX_NB;   // panel width limit
 constexpr int kSb = 8;                    // sub-panel width inside the window
-constexpr int kTileM = 64;                // trailing update tile: 8 warps as 2 x 4,
-constexpr int kTileN = 128;               // warp tile 32 x 32
-constexpr int kStageN = 2 * kTileN;       // trailing columns solved per staging round
-constexpr int kLdb = 36;                  // shared U12 tile stride (== 4 mod 16)
-constexpr int kLdsave = kMaxNb + 2;
+constexpr int kMaxWarps = 16;
+constexpr int kLeftMoves = 2 * kMaxN;     // row moves kept for the columns on the left,
+constexpr int kLeftSegs = 64;             // in at most this many segments
 constexpr int kNone = INT_MAX;            // logical position of a thread's missing row
-static_assert(kMaxN == DP_BATCH_MAX_N, "batched kernel covers n <= DP_BATCH_MAX_N");
-static_assert(kMaxNb == DP_BATCH_MAX_NB, "panel width limit");
-static_assert(kStageN == kThreads, "one staging column per thread");
+
+// One CTA shape: T threads with RPT panel rows each and a register window of
+// NB panel columns; trailing updates in rounds of STAGE columns, the warps
+// WM x WN over tiles of 32 x 32; MINB CTAs per SM.
+template <int T_, int RPT_, int NB_, int STAGE_, int WM_, int MINB_>
+struct Geo {
+  static constexpr int T = T_, RPT = RPT_, NB = NB_, STAGE = STAGE_, WM = WM_, MINB = MINB_;
+  static constexpr int kWarps = T / 32, WN = kWarps / WM;
+  static constexpr int kRows = T * RPT;            // largest order
+  static constexpr int kTileM = 32 * WM, kTileN = 32 * WN;
+  static constexpr int kLdb = NB + 4;              // shared U12 tile stride (== 4 mod 16)
+  static_assert(kWarps % WM == 0 && kWarps <= kMaxWarps && STAGE % kTileN == 0 && STAGE <= T && NB % 16 == 0 && NB <= kMaxNb && kWarps * kRows <= kRows * NB + STAGE * kLdb,
+                "geometry");
+};
 
 struct Params {
   double* base;
@@ -101,20 +106,29 @@ __host__ __device__ inline int bucket_of(int n) {
 }
 
 struct Smem {
-  // dynamic part: P [pr * kMaxNb], then Bs [kStageN * kLdb]
-  double crow[2][kWarps][kSb + 1]; // each warp's candidate row (sub-panel part) and the
+  // dynamic part: P [pr * NB], then Bs [STAGE * kLdb]
+  double crow[2][kMaxWarps][kSb + 1]; // each warp's candidate row (sub-panel part) and the
                                    // reciprocal of its pivot entry, by step parity
-  double rval[2][kWarps];          // each warp's best magnitude (>= 0) and logical row
-  int rkey[2][kWarps];
-  double rsec[2][kWarps];          // each warp's runner-up magnitude (near-tie detector)
-  double psave[kSb][kLdsave];      // the current sub-panel's pivot rows, whole window
-  short mv_dst[2 * kMaxNb];        // the panel's composite row permutation:
-  short mv_src[2 * kMaxNb];        // panel row mv_src[j] moves to mv_dst[j]
-  int mv_count;
-  double fval[kWarps];             // fallback search
-  double fsec[kWarps];
-  int frow[kWarps];
-  int fcol[kWarps];
+  double rval[2][kMaxWarps];          // each warp's best magnitude (>= 0) and logical row
+  int rkey[2][kMaxWarps];
+  double rsec[2][kMaxWarps];          // each warp's runner-up magnitude (near-tie detector)
+  double psave[kSb][kMaxNb + 2];      // the current sub-panel's pivot rows, whole window
+  // The panel's composite row permutation: block row i takes the content of
+  // panel row src_blk[i], panel row ext_dst[j] below the block that of ext_src[j]
+  short src_blk[kMaxNb], ext_dst[kMaxNb], ext_src[kMaxNb];
+  int ext_count;
+  // Row moves still owed to the finished columns on the left (settle_left):
+  // segment t covers the columns [seg_col[t], seg_end[t]); its moves (matrix
+  // row lm_src -> lm_dst, entries [seg_at[t], seg_at[t + 1])) belong to the
+  // columns before seg_col[t].
+  short lm_dst[kLeftMoves], lm_src[kLeftMoves];
+  short seg_col[kLeftSegs], seg_end[kLeftSegs], seg_at[kLeftSegs + 1];
+  int segs;
+  short cur[kMaxN];
+  double fval[kMaxWarps];             // fallback search
+  double fsec[kMaxWarps];
+  int frow[kMaxWarps];
+  int fcol[kMaxWarps];
   int slot;
 };
 
@@ -193,42 +207,33 @@ __device__ __forceinline__ bool offer(double v, int key, double& cv, int& ck, do
   return false;
 }
 
-// Counts one pivot decision of step k in the batch's near-tie counters.
-__device__ __forceinline__ void note_tie(unsigned long long* ties, int k, double best,
-                                         double second) {
-  atomicAdd(ties, 1ull);
-  if (best > 0.0) {
-    if (best - second <= kNearTieC * (double)(k + 1) * 0x1p-53 * best) atomicAdd(ties + 1, 1ull);
-    atomicMax(ties + 2, (unsigned long long)__double_as_longlong(second / best));
-  }
-}
-
 // Factor panel columns [b, b + w) of the n x n matrix A (rows b..n-1).
 // Returns the first step without an acceptable pivot (-1: all w steps done).
 // Writes the panel back in logical row order to A and to P (column stride
-// pr), the step pivots to ipiv, and the rows that moved to s.mv_*.
+// pr), the step pivots to ipiv, and the rows that moved to s.src_blk / s.ext_*.
 //
-// Thread t owns panel rows t and t + 256 (physical rows) and keeps a window
-// of 32 of their columns in registers, x[i][c] = panel column base + c.  The
+// Thread t owns the panel rows t + i T (physical rows) and keeps a window of
+// NB of their columns in registers, x[i][c] = panel column base + c.  The
 // window is factored in sub-panels of kSb columns: kSb unrolled steps of
 // rank-1 updates confined to the sub-panel (one barrier each), then the
 // sub-panel's pivot rows are solved for the rest of the window (U12 =
 // L11^{-1} A12, in shared memory) and the remaining rows take one rank-kSb
 // update; finished columns go to P in physical row order and the window
 // shifts by kSb.  The compiled step body is one sub-panel long.
+template <class G>
 __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int w,
                                           bool positioned, double thr, double* P, int pr,
-                                          Smem& s, int* ipiv, unsigned long long* ties) {
+                                          Smem& s, int* ipiv, DecisionTally& tally) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rows = n - b;
-  double x[kRpt][kMaxNb];
-  int lp[kRpt];
+  double x[G::RPT][G::NB];
+  int lp[G::RPT];
 #pragma unroll
-  for (int i = 0; i < kRpt; ++i) {
-    const int r = tid + i * kThreads;
+  for (int i = 0; i < G::RPT; ++i) {
+    const int r = tid + i * G::T;
     lp[i] = r < rows ? r : kNone;
 #pragma unroll
-    for (int c = 0; c < kMaxNb; ++c)
+    for (int c = 0; c < G::NB; ++c)
       x[i][c] = (r < rows && c < w) ? A[idx(b + r, b + c, lda)] : 0.0;
   }
 
@@ -240,7 +245,7 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
     double pv = 0.0;
 #pragma unroll
     for (int c = 0; c < kSb; ++c)
-      if (c == j) pv = ci ? x[kRpt - 1][c] : x[0][c];
+      if (c == j) pv = ci ? x[G::RPT - 1][c] : x[0][c];
     const double rinv = 1.0 / pv;
     double wv;
     int wk;
@@ -251,7 +256,7 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
       if (wk != kNone) {
 #pragma unroll
         for (int c = 0; c < kSb; ++c)
-          if (c >= j) s.crow[par][warp][c] = ci ? x[kRpt - 1][c] : x[0][c];
+          if (c >= j) s.crow[par][warp][c] = ci ? x[G::RPT - 1][c] : x[0][c];
         s.crow[par][warp][kSb] = rinv;
       }
       s.rval[par][warp] = wv;
@@ -264,7 +269,7 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
     double cv = 0.0, cs = 0.0;
     int ck = kNone, ci = 0;
 #pragma unroll
-    for (int i = 0; i < kRpt; ++i) {
+    for (int i = 0; i < G::RPT; ++i) {
       if (lp[i] == kNone || lp[i] < first) continue;
       // a placed pivot (after a fallback) is the only candidate of its step
       if (placed && lp[i] != first) continue;
@@ -275,7 +280,7 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
   };
 
   first_candidate(0, positioned);
-  if (tid == 0) s.mv_count = 0;
+  if (tid == 0) s.ext_count = 0;
   __syncthreads();
 
   int stop = -1;
@@ -289,19 +294,19 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
       const int st = base + j, par = st & 1;
       double bv;
       int bk;
-      warp_best(s.rval[par][lane & (kWarps - 1)], s.rkey[par][lane & (kWarps - 1)], bv, bk);
+      warp_best(s.rval[par][lane & (G::kWarps - 1)], s.rkey[par][lane & (G::kWarps - 1)], bv, bk);
       // the warp that offered the winner (keys of real candidates are unique)
-      const int bw = max(0, __ffs(__ballot_sync(0xffffffffu, lane < kWarps && bk != kNone &&
+      const int bw = max(0, __ffs(__ballot_sync(0xffffffffu, lane < G::kWarps && bk != kNone &&
                                                                 s.rkey[par][lane] == bk)) - 1);
       const bool placed = positioned && st == 0;
       if (!placed) {
-        // runner-up over the warps (lanes >= kWarps repeat lanes < kWarps)
-        const int q = lane & (kWarps - 1);
+        // runner-up over the warps (lanes >= G::kWarps repeat lanes < G::kWarps)
+        const int q = lane & (G::kWarps - 1);
         const double bs = warp_max_pos((bk != kNone && s.rkey[par][q] == bk)
                                            ? s.rsec[par][q]
                                            : (s.rkey[par][q] != kNone ? s.rval[par][q]
                                                                       : s.rsec[par][q]));
-        if (tid == 0) note_tie(ties, b + st, bk != kNone ? bv : 0.0, bs);
+        if (tid == 0) tally.note(b + st, bk != kNone ? bv : 0.0, bs);
       }
       if (!placed && !(bv > thr)) {
         stop = st;
@@ -315,11 +320,11 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
       double cv = 0.0, cs = 0.0;
       int ck = kNone, ci = 0;
 #pragma unroll
-      for (int i = 0; i < kRpt; ++i) {
+      for (int i = 0; i < G::RPT; ++i) {
         if (lp[i] == p) {
           lp[i] = st;  // the pivot row: keep its window for the U12 solve
 #pragma unroll
-          for (int g = 0; g < kMaxNb / kSb; ++g)
+          for (int g = 0; g < G::NB / kSb; ++g)
             if (base + g * kSb < w) {
 #pragma unroll
               for (int c = g * kSb; c < (g + 1) * kSb; ++c) s.psave[j][c] = x[i][c];
@@ -346,7 +351,7 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
     const int rest = w - base - kSb;
     __syncthreads();  // psave complete
     if (kd > 0 && rest > 0) {
-      for (int c = kSb + tid; c < kSb + rest; c += kThreads)
+      for (int c = kSb + tid; c < kSb + rest; c += G::T)
         for (int j = 1; j < kd; ++j) {
           double u = s.psave[j][c];
           for (int t = 0; t < j; ++t) u = fma(-s.psave[j][t], s.psave[t][c], u);
@@ -354,19 +359,19 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
         }
       __syncthreads();
 #pragma unroll
-      for (int i = 0; i < kRpt; ++i) {
+      for (int i = 0; i < G::RPT; ++i) {
         if (lp[i] == kNone || lp[i] < base) continue;
         if (lp[i] < base + kd) {  // a pivot row of this sub-panel takes its U12 row
           const double* u = s.psave[lp[i] - base];
 #pragma unroll
-          for (int g = 1; g < kMaxNb / kSb; ++g)
+          for (int g = 1; g < G::NB / kSb; ++g)
             if (base + g * kSb < w) {
 #pragma unroll
               for (int c = g * kSb; c < (g + 1) * kSb; ++c) x[i][c] = u[c];
             }
         } else {
 #pragma unroll
-          for (int g = 1; g < kMaxNb / kSb; ++g)
+          for (int g = 1; g < G::NB / kSb; ++g)
             if (base + g * kSb < w) {
 #pragma unroll
               for (int t = 0; t < kSb; ++t)
@@ -383,16 +388,16 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
     if (stop >= 0) break;
     // finished sub-panel columns to P (physical rows); shift the window
 #pragma unroll
-    for (int i = 0; i < kRpt; ++i) {
+    for (int i = 0; i < G::RPT; ++i) {
       if (lp[i] == kNone) continue;
-      double* pc = P + tid + i * kThreads + (size_t)base * pr;
+      double* pc = P + tid + i * G::T + (size_t)base * pr;
 #pragma unroll
       for (int c = 0; c < kSb; ++c)
         if (c < sw) pc[c * pr] = x[i][c];
 #pragma unroll
-      for (int c = 0; c < kMaxNb - kSb; ++c) x[i][c] = x[i][c + kSb];
+      for (int c = 0; c < G::NB - kSb; ++c) x[i][c] = x[i][c + kSb];
 #pragma unroll
-      for (int c = kMaxNb - kSb; c < kMaxNb; ++c) x[i][c] = 0.0;
+      for (int c = G::NB - kSb; c < G::NB; ++c) x[i][c] = 0.0;
     }
     base += kSb;
     if (base < w) {
@@ -402,121 +407,216 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
   }
   // the window's remaining columns to P (physical rows)
 #pragma unroll
-  for (int i = 0; i < kRpt; ++i) {
+  for (int i = 0; i < G::RPT; ++i) {
     if (lp[i] == kNone) continue;
-    double* pc = P + tid + i * kThreads;
+    double* pc = P + tid + i * G::T;
 #pragma unroll
-    for (int c = 0; c < kMaxNb; ++c)
+    for (int c = 0; c < G::NB; ++c)
       if (base + c < w) pc[(size_t)(base + c) * pr] = x[i][c];
   }
   __syncthreads();
   // rows to their logical positions, in P and in the matrix
 #pragma unroll
-  for (int i = 0; i < kRpt; ++i) {
+  for (int i = 0; i < G::RPT; ++i) {
     if (lp[i] == kNone) continue;
-    const double* pc = P + tid + i * kThreads;
+    const double* pc = P + tid + i * G::T;
 #pragma unroll
-    for (int c = 0; c < kMaxNb; ++c)
+    for (int c = 0; c < G::NB; ++c)
       if (c < w) x[i][c] = pc[c * pr];
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kRpt; ++i) {
+  for (int i = 0; i < G::RPT; ++i) {
     if (lp[i] == kNone) continue;
-    const int r = lp[i], phys = tid + i * kThreads;
+    const int r = lp[i], phys = tid + i * G::T;
 #pragma unroll
-    for (int c = 0; c < kMaxNb; ++c)
+    for (int c = 0; c < G::NB; ++c)
       if (c < w) {
         A[idx(b + r, b + c, lda)] = x[i][c];
         if (r != phys) P[r + c * pr] = x[i][c];
       }
-    if (r != phys) {  // at most two rows per executed step move
-      const int j = atomicAdd(&s.mv_count, 1);
-      s.mv_dst[j] = (short)r;
-      s.mv_src[j] = (short)phys;
+    if (r < w) {
+      s.src_blk[r] = (short)phys;
+    } else if (r != phys) {  // at most one row per executed step
+      const int j = atomicAdd(&s.ext_count, 1);
+      s.ext_dst[j] = (short)r;
+      s.ext_src[j] = (short)phys;
     }
   }
   return stop;
 }
 
-// The panel's row permutation on every column outside it ([0, b) and
-// [b + w, n)): four lanes per column gather all moved rows into registers
-// (lane h takes the moves j == h mod 4), meet at a warp barrier, then store
-// them at their destinations - no dependent swap chain.
-__device__ __forceinline__ void permute_outside(double* A, int lda, int n, int b, int w,
-                                                const Smem& s) {
-  const int cnt = s.mv_count;
-  if (cnt == 0) return;
-  const int h = threadIdx.x & 3;
-  const int total = n - w;
-  for (int t0 = 0; t0 < total; t0 += kThreads / 4) {  // the same trip count for every lane
-    const int t = t0 + ((int)threadIdx.x >> 2);
-    const bool on = t < total;
-    double* col = A + idx(b, on ? (t < b ? t : t + w) : 0, lda);
-    double v[kMaxNb / 2];
-#pragma unroll
-    for (int q = 0; q < kMaxNb / 2; ++q) {
-      const int j = 4 * q + h;
-      if (on && j < cnt) v[q] = col[s.mv_src[j]];
+// The row moves kept for the finished columns, applied: each column is read
+// and written once, coalesced, through a buffer of its warp in shared memory
+// (`buf`, n doubles a warp: P and the U12 tile behind it), instead of 2 nb
+// scattered elements per panel and column (n = 512: 0.5 of 3.0 ms).  From the
+// last segment back, s.cur holds the composite of the moves after the segment:
+// position r of its columns takes row cur[r].
+template <class G>
+__device__ __forceinline__ void settle_left(double* A, int lda, int n, double* buf, Smem& s) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* const mine = buf + warp * n;
+  __syncthreads();  // the moves are listed, buf is free
+  const int segs = s.segs;
+  for (int r = tid; r < n; r += G::T) s.cur[r] = (short)r;
+  __syncthreads();
+  for (int t = segs - 1; t >= 0; --t) {
+    const int c0 = s.seg_col[t], c1 = s.seg_end[t];
+    if (t + 1 < segs)
+      for (int c = c0 + warp; c < c1; c += G::kWarps) {
+        double* const col = A + idx(0, c, lda);
+        for (int r = c1 + lane; r < n; r += 32) mine[r] = col[r];
+        __syncwarp();
+        for (int r = c1 + lane; r < n; r += 32) {
+          const int from = s.cur[r];
+          if (from != r) col[r] = mine[from];
+        }
+        __syncwarp();
+      }
+    // cur <- (this segment's moves) o cur; a moved row is looked up in the
+    // list through `back`, the moves' sources by position
+    const int m0 = s.seg_at[t], m1 = s.seg_at[t + 1];
+    if (t == 0 || m0 == m1) continue;
+    __syncthreads();  // the columns have read cur, and buf is free
+    short* const back = reinterpret_cast<short*>(buf);
+    for (int r = tid; r < n; r += G::T) back[r] = (short)r;
+    __syncthreads();
+    for (int m = m0 + tid; m < m1; m += G::T) back[s.lm_dst[m]] = s.lm_src[m];
+    __syncthreads();
+    for (int r = tid; r < n; r += G::T) s.cur[r] = back[s.cur[r]];
+    __syncthreads();
+  }
+  __syncthreads();
+  if (tid == 0 && segs > 0) {  // the columns settled so far are owed what comes after
+    s.seg_end[0] = s.seg_end[segs - 1];
+    s.seg_col[0] = 0;
+    s.seg_at[0] = s.seg_at[1] = 0;
+    s.segs = 1;
+  }
+  __syncthreads();
+}
+
+// Adds the segment of columns [c0, c1) whose `ext` and block moves (a panel's,
+// rows from b) the columns before c0 are still owed; every thread calls it.
+template <class G>
+__device__ __forceinline__ void keep_panel_moves(int b, int w, int c1, Smem& s) {
+  // one warp, in list order (the entries' order within a segment is free)
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int at = s.seg_at[s.segs];
+    const bool blk = lane < w && s.src_blk[lane] != lane;
+    const unsigned mb = __ballot_sync(~0u, blk);
+    if (blk) {
+      const int m = at + __popc(mb & ((1u << lane) - 1u));
+      s.lm_dst[m] = (short)(b + lane);
+      s.lm_src[m] = (short)(b + s.src_blk[lane]);
+    }
+    at += __popc(mb);
+    const int ext = s.ext_count;
+    if (lane < ext) {
+      s.lm_dst[at + lane] = (short)(b + s.ext_dst[lane]);
+      s.lm_src[at + lane] = (short)(b + s.ext_src[lane]);
     }
     __syncwarp();
-#pragma unroll
-    for (int q = 0; q < kMaxNb / 2; ++q) {
-      const int j = 4 * q + h;
-      if (on && j < cnt) col[s.mv_dst[j]] = v[q];
+    if (lane == 0) {
+      const int t = s.segs;
+      s.seg_col[t] = (short)b;
+      s.seg_end[t] = (short)c1;
+      s.seg_at[t + 1] = (short)(at + ext);
+      s.segs = t + 1;
     }
   }
 }
 
-// Right of a panel that executed `kd` steps at [b, b + kd), its row
-// permutation already applied: for the columns [c0, n), U12 = L11^{-1}
+// Right of a panel of w columns that executed `kd` steps at [b, b + kd): for
+// the columns [c0, n), the panel's row permutation, U12 = L11^{-1}
 // A(b:b+kd, :) (written back) and A(b+kd:n, :) -= L21 U12, with L11 / L21 the
-// shared panel P.  TERMS = 0: the product in FP64 (DMMA); TERMS = 2 / 3: the
+// shared panel P.  The permutation is part of the staging: a group of NB lanes
+// gathers a column's new block rows into the shared tile and carries the
+// displaced rows below the block to their places, all of a column's loads
+// before its stores; the solve then runs from shared memory with a thread per
+// column, and the block rows go back coalesced.  (As passes of their own over
+// global memory, the permutation four lanes a column and the solve a thread a
+// column, they took 0.5 and 0.9 of the 3.0 ms of an n = 512 matrix: every
+// element access of a warp was a transaction of its own.)  TERMS = 0: the product in FP64 (DMMA); TERMS = 2 / 3: the
 // BF16 split product (3 / 6 products, FP32 accumulation), subtracted in FP64.
-template <int TERMS>
-__device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b, int kd, int c0,
-                                                const double* P, int pr, double* Bs) {
+template <class G, int TERMS>
+__device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b, int w, int kd,
+                                                int c0, const double* P, int pr, double* Bs,
+                                                const Smem& s) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = warp >> 2, wn = warp & 3;
+  const int wm = warp / G::WN, wn = warp % G::WN;
   const int row0 = b + kd;
   const int M = n - row0, N = n - c0;
   const int kp = (kd + 3) & ~3;
   const double* L21 = P + kd;  // panel rows kd.. = matrix rows row0..
-  for (int n0 = 0; n0 < N; n0 += kStageN) {
-    const int ns = min(kStageN, N - n0);
+  for (int n0 = 0; n0 < N; n0 += G::STAGE) {
+    const int ns = min(G::STAGE, N - n0);
     __syncthreads();  // Bs is free
-    {
-      double* bcol = Bs + tid * kLdb;
-      if (tid < ns) {
-        double* col = A + idx(0, c0 + n0 + tid, lda);
-        double u[kMaxNb];
+    constexpr int kLanes = G::NB;               // lanes per column
+    constexpr int kCols = 32 / kLanes;          // columns per warp and pass
+    constexpr int kUnroll = 4;
+    const int li = lane % kLanes, lc = lane / kLanes;
+    const int ext = s.ext_count;
+    for (int q0 = warp * kCols * kUnroll; q0 < G::STAGE; q0 += G::kWarps * kCols * kUnroll) {
+      double blk[kUnroll], low[kUnroll];
 #pragma unroll
-        for (int i = 0; i < kMaxNb; ++i) u[i] = i < kd ? col[b + i] : 0.0;
+      for (int u = 0; u < kUnroll; ++u) {
+        const int c = q0 + u * kCols + lc;
+        const double* col = A + idx(b, c0 + n0 + c, lda);
+        blk[u] = (c < ns && li < w) ? col[s.src_blk[li]] : 0.0;
+        low[u] = (c < ns && li < ext) ? col[s.ext_src[li]] : 0.0;
+      }
 #pragma unroll
-        for (int j = 0; j < kMaxNb - 1; ++j) {
-          if (j >= kd) break;
-          const double uj = u[j];
+      for (int u = 0; u < kUnroll; ++u) Bs[(q0 + u * kCols + lc) * G::kLdb + li] = blk[u];
+      __syncwarp();  // the pass's columns are read
 #pragma unroll
-          for (int i = j + 1; i < kMaxNb; ++i)
-            if (i < kd) u[i] = fma(-P[i + j * pr], uj, u[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < kMaxNb; ++i)
-          if (i < kp) {
-            if (i < kd) col[b + i] = u[i];
-            bcol[i] = i < kd ? u[i] : 0.0;
-          }
-      } else {
-        for (int i = 0; i < kp; ++i) bcol[i] = 0.0;
+      for (int u = 0; u < kUnroll; ++u) {
+        const int c = q0 + u * kCols + lc;
+        if (c < ns && li < ext) A[idx(b + s.ext_dst[li], c0 + n0 + c, lda)] = low[u];
       }
     }
     __syncthreads();
-    for (int h = 0; h * kTileN < ns; ++h) {
-      const int nc = min(kTileN, ns - h * kTileN);
-      const double* Bh = Bs + h * kTileN * kLdb;
-      double* C = A + idx(row0, c0 + n0 + h * kTileN, lda);
-      for (int m0 = 0; m0 < M; m0 += kTileM) {
+    if (tid < ns) {
+      double* bcol = Bs + tid * G::kLdb;
+      double u[G::NB];
+#pragma unroll
+      for (int i = 0; i < G::NB; i += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(bcol + i);
+        u[i] = v.x;
+        u[i + 1] = v.y;
+      }
+#pragma unroll
+      for (int j = 0; j < G::NB - 1; ++j) {
+        if (j >= kd) break;
+        const double uj = u[j];
+        const double2* pj = reinterpret_cast<const double2*>(P + j * pr);
+#pragma unroll
+        for (int i = j & ~1; i < G::NB; i += 2)
+          if (i < kd) {  // (uniform; pairs: row i <= j and, at the end, row kd are left alone)
+            const double2 l = pj[i / 2];
+            if (i > j) u[i] = fma(-l.x, uj, u[i]);
+            if (i + 1 > j && i + 1 < kd) u[i + 1] = fma(-l.y, uj, u[i + 1]);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < G::NB; i += 2)
+        *reinterpret_cast<double2*>(bcol + i) = make_double2(u[i], u[i + 1]);
+    }
+    __syncthreads();
+    for (int q = warp * kCols; q < ns; q += G::kWarps * kCols) {
+      const int c = q + lc;
+      double* e = Bs + c * G::kLdb + li;
+      if (c < ns && li < w) A[idx(b + li, c0 + n0 + c, lda)] = *e;
+      if (li >= kd) *e = 0.0;  // not part of the product
+    }
+    __syncthreads();
+    for (int h = 0; h * G::kTileN < ns; ++h) {
+      const int nc = min(G::kTileN, ns - h * G::kTileN);
+      const double* Bh = Bs + h * G::kTileN * G::kLdb;
+      double* C = A + idx(row0, c0 + n0 + h * G::kTileN, lda);
+      for (int m0 = 0; m0 < M; m0 += G::kTileM) {
         const int rb = m0 + wm * 32;
         if (rb >= M) continue;  // warp-uniform; no barrier inside this loop
         double cf[2][4][4];
@@ -530,14 +630,9 @@ __device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b
               const int c = wn * 32 + ni * 8 + 2 * t + (v & 1);
               cf[mi][ni][v] = (r < M && c < nc) ? C[idx(r, c, lda)] : 0.0;
             }
-        double acc[2][4][4];
         if constexpr (TERMS == 0) {
-#pragma unroll
-          for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-              for (int v = 0; v < 4; ++v) acc[mi][ni][v] = 0.0;
+          // C itself is the accumulator (and -L21 the operand): half the
+          // registers of a separate sum, which two CTAs per SM need
           for (int k0 = 0; k0 < kp; k0 += 4) {
             const int kk = k0 + t;
             const bool kok = kk < kd;
@@ -545,16 +640,16 @@ __device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi) {
               const int r = rb + mi * 16 + g;
-              a[mi][0] = (kok && r < M) ? L21[r + kk * pr] : 0.0;
-              a[mi][1] = (kok && r + 8 < M) ? L21[r + 8 + kk * pr] : 0.0;
+              a[mi][0] = (kok && r < M) ? -L21[r + kk * pr] : 0.0;
+              a[mi][1] = (kok && r + 8 < M) ? -L21[r + 8 + kk * pr] : 0.0;
             }
             double bf[4];
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) bf[ni] = Bh[(wn * 32 + ni * 8 + g) * kLdb + kk];
+            for (int ni = 0; ni < 4; ++ni) bf[ni] = Bh[(wn * 32 + ni * 8 + g) * G::kLdb + kk];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-              for (int ni = 0; ni < 4; ++ni) mma_f64(acc[mi][ni], a[mi][0], a[mi][1], bf[ni]);
+              for (int ni = 0; ni < 4; ++ni) mma_f64(cf[mi][ni], a[mi][0], a[mi][1], bf[ni]);
           }
         } else {
           // m16n8k16 fragments: A (row r, k) at r = g / g + 8 and k = 2t, 2t + 1,
@@ -585,7 +680,7 @@ __device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
-                const double* bc = Bh + (wn * 32 + ni * 8 + g) * kLdb;
+                const double* bc = Bh + (wn * 32 + ni * 8 + g) * G::kLdb;
                 const int kk = k0 + 2 * t + 8 * h;
                 __nv_bfloat16 lo[TERMS], hi[TERMS];
                 split_pieces<TERMS>(kk < kd ? bc[kk] : 0.0, lo);
@@ -607,7 +702,7 @@ __device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b
 #pragma unroll
             for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
-              for (int v = 0; v < 4; ++v) acc[mi][ni][v] = (double)facc[mi][ni][v];
+              for (int v = 0; v < 4; ++v) cf[mi][ni][v] -= (double)facc[mi][ni][v];
         }
 #pragma unroll
         for (int mi = 0; mi < 2; ++mi)
@@ -617,7 +712,7 @@ __device__ __forceinline__ void trailing_update(double* A, int lda, int n, int b
             for (int v = 0; v < 4; ++v) {
               const int r = rb + mi * 16 + g + 8 * (v >> 1);
               const int c = wn * 32 + ni * 8 + 2 * t + (v & 1);
-              if (r < M && c < nc) C[idx(r, c, lda)] = cf[mi][ni][v] - acc[mi][ni][v];
+              if (r < M && c < nc) C[idx(r, c, lda)] = cf[mi][ni][v];
             }
       }
     }
@@ -630,6 +725,7 @@ __device__ __forceinline__ bool better2(double va, int ca, int ra, double vb, in
 
 // 2-D argmax over the active block A(k:n, k:n): larger magnitude, then the
 // smaller column, then the smaller row; NaN never wins.
+template <class G>
 __device__ __forceinline__ void active_argmax(const double* A, int lda, int n, int k, Smem& s,
                                               double& bv, int& br, int& bc, double& bs) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -637,7 +733,7 @@ __device__ __forceinline__ void active_argmax(const double* A, int lda, int n, i
   int r0 = INT_MAX, c0 = INT_MAX;
   const int rows = n - k;
   for (int c = k; c < n; ++c)
-    for (int r = tid; r < rows; r += kThreads) {
+    for (int r = tid; r < rows; r += G::T) {
       const double v = fabs(A[idx(k + r, c, lda)]);
       if (v > v0) {  // (column, row) increase along this thread's scan
         s0 = fmax(s0, v0);
@@ -675,7 +771,7 @@ __device__ __forceinline__ void active_argmax(const double* A, int lda, int n, i
   bs = s.fsec[0];
   br = s.frow[0];
   bc = s.fcol[0];
-  for (int q = 1; q < kWarps; ++q)
+  for (int q = 1; q < G::kWarps; ++q)
     if (better2(s.fval[q], s.fcol[q], s.frow[q], bv, bc, br)) {
       bs = fmax(s.fsec[q], bv);
       bv = s.fval[q];
@@ -686,54 +782,68 @@ __device__ __forceinline__ void active_argmax(const double* A, int lda, int n, i
     }
 }
 
-template <int TERMS>
+template <class G, int TERMS>
 __device__ __forceinline__ void getrf_one(double* A, int n, int* ipiv, int* jpiv, int* info,
                                           int nb, double thr, double* P, int pr, double* Bs,
-                                          Smem& s, unsigned long long* ties) {
+                                          Smem& s, DecisionTally& tally) {
   const int tid = threadIdx.x;
   const int lda = n;
-  for (int i = tid; i < n; i += kThreads) ipiv[i] = jpiv[i] = i;
-  if (tid == 0) *info = n;
+  for (int i = tid; i < n; i += G::T) ipiv[i] = jpiv[i] = i;
+  if (tid == 0) {
+    *info = n;
+    s.segs = 0;
+    s.seg_at[0] = 0;
+  }
   int b = 0;
   bool positioned = false;
   while (b < n) {
     const int w = min(nb, n - b), e = b + w;
-    __syncthreads();  // P, Bs, the move list and the records are settled
-    const int stop = panel_regs(A, n, lda, b, w, positioned, thr, P, pr, s, ipiv, ties);
+    __syncthreads();  // P, Bs, the move lists and the records are settled
+    if (s.segs + 3 > kLeftSegs || s.seg_at[s.segs] + 2 * kMaxNb + 2 > kLeftMoves)
+      settle_left<G>(A, lda, n, P, s);
+    const int stop = panel_regs<G>(A, n, lda, b, w, positioned, thr, P, pr, s, ipiv, tally);
     positioned = false;
     __syncthreads();  // panel written back, move list complete
-    permute_outside(A, lda, n, b, w, s);
+    keep_panel_moves<G>(b, w, stop < 0 ? e : b + stop, s);
     if (stop < 0) {
-      if (e < n) trailing_update<TERMS>(A, lda, n, b, w, e, P, pr, Bs);
+      if (e < n) trailing_update<G, TERMS>(A, lda, n, b, w, w, e, P, pr, Bs, s);
       b = e;
       continue;
     }
     // column k has no acceptable pivot: bring the columns right of the panel
     // up to date for the executed steps, then search the whole active block
     const int k = b + stop;
-    if (e < n && stop > 0) trailing_update<TERMS>(A, lda, n, b, stop, e, P, pr, Bs);
+    if (e < n && stop > 0) trailing_update<G, TERMS>(A, lda, n, b, w, stop, e, P, pr, Bs, s);
     __syncthreads();
     double bv, bs;
     int br, bc;
-    active_argmax(A, lda, n, k, s, bv, br, bc, bs);
-    if (tid == 0) note_tie(ties, k, bv > 0.0 ? bv : 0.0, bv > 0.0 ? bs : 0.0);
+    active_argmax<G>(A, lda, n, k, s, bv, br, bc, bs);
+    if (tid == 0) tally.note(k, bv > 0.0 ? bv : 0.0, bv > 0.0 ? bs : 0.0);
     if (!(bv > thr)) {
       if (tid == 0) *info = k;
-      return;
+      break;
     }
     if (tid == 0) {
       ipiv[k] = br;
       jpiv[k] = bc;
+      if (br != k) {  // the columns before k are owed the row swap
+        const int t = s.segs, at = s.seg_at[t];
+        s.lm_dst[at] = s.lm_src[at + 1] = (short)k;
+        s.lm_src[at] = s.lm_dst[at + 1] = (short)br;
+        s.seg_col[t] = s.seg_end[t] = (short)k;
+        s.seg_at[t + 1] = (short)(at + 2);
+        s.segs = t + 1;
+      }
     }
     if (br != k)
-      for (int c = tid; c < n; c += kThreads) {
+      for (int c = k + tid; c < n; c += G::T) {
         const double tmp = A[idx(k, c, lda)];
         A[idx(k, c, lda)] = A[idx(br, c, lda)];
         A[idx(br, c, lda)] = tmp;
       }
     __syncthreads();
     if (bc != k)
-      for (int r = tid; r < n; r += kThreads) {
+      for (int r = tid; r < n; r += G::T) {
         const double tmp = A[idx(r, k, lda)];
         A[idx(r, k, lda)] = A[idx(r, bc, lda)];
         A[idx(r, bc, lda)] = tmp;
@@ -741,14 +851,18 @@ __device__ __forceinline__ void getrf_one(double* A, int n, int* ipiv, int* jpiv
     b = k;
     positioned = true;
   }
+  settle_left<G>(A, lda, n, P, s);
 }
 
-template <int TERMS>
-__global__ void __launch_bounds__(kThreads, 1) batched_getrf_kernel(Params p) {
+template <class G, int TERMS>
+__global__ void __launch_bounds__(G::T, G::MINB) batched_getrf_kernel(Params p) {
+  // the next size class's CTAs may take the SMs this one leaves free
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(16) double dsm[];
   __shared__ Smem s;
   double* P = dsm;
-  double* Bs = dsm + (size_t)p.pr * kMaxNb;
+  double* Bs = dsm + (size_t)p.pr * G::NB;
+  DecisionTally tally;
   while (true) {
     __syncthreads();  // s.slot is free
     if (threadIdx.x == 0) s.slot = atomicAdd(p.queue, 1);
@@ -758,11 +872,18 @@ __global__ void __launch_bounds__(kThreads, 1) batched_getrf_kernel(Params p) {
     const int i = p.order[slot];
     const int n = p.ns[i];
     const int bk = bucket_of(n);  // selected without indexing the parameter array
-    const int nb = bk == 0 ? p.nb_bucket[0] : bk == 1 ? p.nb_bucket[1] : bk == 2 ? p.nb_bucket[2]
-                                                                                 : p.nb_bucket[3];
-    getrf_one<TERMS>(p.base + p.offsets[i], n, p.ipiv + p.rec_offsets[i], p.jpiv + p.rec_offsets[i],
-              p.info + i, nb, p.threshold, P, p.pr, Bs, s, p.ties);
+    const int nb = min(G::NB, bk == 0   ? p.nb_bucket[0]
+                              : bk == 1 ? p.nb_bucket[1]
+                              : bk == 2 ? p.nb_bucket[2]
+                                        : p.nb_bucket[3]);
+    getrf_one<G, TERMS>(p.base + p.offsets[i], n, p.ipiv + p.rec_offsets[i],
+                        p.jpiv + p.rec_offsets[i], p.info + i, nb, p.threshold, P, p.pr, Bs, s,
+                        tally);
   }
+  if (threadIdx.x == 0) tally.flush(p.ties, p.ties + 1, p.ties + 2);
+  // the launch ends no earlier than the classes before it: what follows on the
+  // stream waits for the last class only
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // One panel of the blocked LU (PanelParams, the same contract as
@@ -772,7 +893,8 @@ __global__ void __launch_bounds__(kThreads, 1) batched_getrf_kernel(Params p) {
 // one CTA barrier per step and no cluster exchange (panel_regs, the batched
 // kernel's panel).  Afterwards the composite row permutation is written as
 // the swap lists the laswp kernel applies outside the panel.
-__global__ void __launch_bounds__(kThreads, 1) panel_small_kernel(PanelParams p) {
+template <class G>
+__global__ void __launch_bounds__(G::T, 1) panel_small_kernel(PanelParams p) {
   // every thread reads the same word before any barrier or state write
   if (p.gated && p.state->stop_k >= 0) return;
   extern __shared__ __align__(16) double dsm[];
@@ -780,46 +902,80 @@ __global__ void __launch_bounds__(kThreads, 1) panel_small_kernel(PanelParams p)
   const int tid = threadIdx.x, lane = tid & 31;
   const int b = p.begin, w = p.end - p.begin;
   const int pr = panel_ld(p.m - b);
-  if (tid == 0) {
-    p.state->stop_k = -1;
-    p.state->swap_count = 0;
-    p.state->block_changed = 0;
-  }
-  const int stop = panel_regs(p.a, p.m, (int)p.lda, b, w, p.positioned != 0, p.threshold, dsm, pr,
-                              s, p.ipiv, &p.state->ties_checked);
-  __syncthreads();  // rows written back, move list complete
-  for (int i = tid; i < w; i += kThreads) p.swap_block[i] = b + i;
-  __syncthreads();
-  const int cnt = s.mv_count;
-  int changed = 0;
-  for (int j0 = 0; j0 < cnt; j0 += kThreads) {  // whole warps: one atomic per warp
-    const int j = j0 + tid;
-    const bool on = j < cnt;
-    const int dst = on ? s.mv_dst[j] : 0, src = on ? s.mv_src[j] : 0;
-    if (on && dst < w) {
-      p.swap_block[dst] = b + src;
-      ++changed;
+  DecisionTally tally;
+  if (tid == 0) p.state->stop_k = -1;
+  const int stop = panel_regs<G>(p.a, p.m, (int)p.lda, b, w, p.positioned != 0, p.threshold, dsm, pr,
+                              s, p.ipiv, tally);
+  __syncthreads();  // rows written back, move lists complete
+  if (tid < 32) {
+    const int ext = s.ext_count;
+    const bool moved = lane < w && s.src_blk[lane] != lane;
+    if (lane < w) p.swap_block[lane] = b + s.src_blk[lane];
+    if (lane < ext) {
+      p.swap_extra[2 * lane + 0] = b + s.ext_dst[lane];
+      p.swap_extra[2 * lane + 1] = b + s.ext_src[lane];
     }
-    const bool below = on && dst >= w;
-    const unsigned bal = __ballot_sync(0xffffffffu, below);
-    if (bal) {
-      int slot = 0;
-      if (lane == 0) slot = atomicAdd(&p.state->swap_count, __popc(bal));
-      slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(bal & ((1u << lane) - 1u));
-      if (below) {
-        p.swap_extra[2 * slot + 0] = b + dst;
-        p.swap_extra[2 * slot + 1] = b + src;
-      }
+    const int changed = __popc(__ballot_sync(~0u, moved));
+    if (lane == 0) {
+      p.state->swap_count = ext;
+      p.state->block_changed = changed;
+      if (stop >= 0) p.state->stop_k = b + stop;
+      tally.flush(p.state);
     }
   }
-  changed = __reduce_add_sync(0xffffffffu, changed);
-  if (lane == 0 && changed) atomicAdd(&p.state->block_changed, changed);
-  if (tid == 0 && stop >= 0) p.state->stop_k = b + stop;
 }
 
+template <class G>
 size_t dynamic_smem(int max_n) {
-  return ((size_t)panel_ld(std::max(max_n, 1)) * kMaxNb + (size_t)kStageN * kLdb) *
+  return ((size_t)panel_ld(std::max(max_n, 1)) * G::NB + (size_t)G::STAGE * G::kLdb) *
          sizeof(double);
+}
+
+// Size classes, by order.  A matrix keeps one CTA busy with chains (a barrier a
+// column, trips to L2 between phases), so the SM has to hold several: the class
+// takes the fewest threads that give each row one, a window of 16 columns (a
+// row's 32 registers leave room for 128 a thread in all) and U12 tiles sized
+// for 2, 4 and 7 CTAs per SM.  2048 matrices of a class, one CTA shape of 256
+// threads for all (two rows a thread, 32 columns, one CTA per SM) -> these:
+// [32, 64] 2.29 -> 0.47 ms, [65, 128] 4.49 -> 1.22, [129, 256] 8.04 -> 3.52,
+// [257, 512] 26.6 -> 17.6.  Measured slower: 32-column windows (up to 512:
+// 20.6, up to 256: 5.3, up to 128: 2.0), 256 threads of two rows for the
+// largest class (18.9; with two CTAs per SM 21.5), tiles of 16 x 32 with the
+// next one's loads in flight (19.1).
+using Geo3 = Geo<512, 1, 16, 256, 4, 1>;
+using Geo2 = Geo<256, 1, 16, 128, 2, 2>;
+using Geo1 = Geo<128, 1, 16, 128, 2, 4>;
+using Geo0 = Geo<64, 1, 16, 64, 1, 7>;
+
+// Panels of the blocked LU: a row per thread (STAGE and the warp grid unused).
+template <int T>
+using PanelGeo = Geo<T, 1, kMaxNb, 32 * (T / 64), 2, 1>;
+
+int class_of(int n) { return n <= 64 ? 0 : n <= 128 ? 1 : n <= 256 ? 2 : 3; }
+
+template <class G>
+int launch_class(Params p, int max_n, int sms, int terms, bool behind, cudaStream_t st) {
+  const void* fn = terms == 3   ? (const void*)batched_getrf_kernel<G, 3>
+                   : terms == 2 ? (const void*)batched_getrf_kernel<G, 2>
+                                : (const void*)batched_getrf_kernel<G, 0>;
+  p.pr = panel_ld(max_n);
+  const size_t smem = dynamic_smem<G>(max_n);
+  if (!dp::ensure_smem(fn, smem)) return DP_CUDA_FAILURE;
+  const int per_sm = dp::occupancy_once(fn, G::T, smem);
+  if (per_sm < 1) return DP_CUDA_FAILURE;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(std::max(1, std::min(p.count, sms * per_sm)));
+  cfg.blockDim = dim3(G::T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = behind ? 1 : 0;
+  dp::note_launch();
+  void* args[] = {&p};
+  return cudaLaunchKernelExC(&cfg, fn, args) == cudaSuccess ? DP_SUCCESS : DP_CUDA_FAILURE;
 }
 
 // N(0,1) by the Box-Muller transform of two hashed uniforms (autotuner inputs).
@@ -850,7 +1006,7 @@ __global__ void fill_normal_kernel(double* x, long long len, uint64_t seed) {
 struct dp_batch {
   int device = 0;
   int count = 0;
-  int max_n = 0;
+  dp::batch::Classes classes;
   int sms = 0;
   long long total_elements = 0;
   long long total_records = 0;
@@ -878,7 +1034,7 @@ bool valid_batch_options(const dp_batch_options* o) {
 }
 
 int launch(dp_batch* bp, double* d_base, int* d_ipiv, int* d_jpiv, int* d_info, cudaStream_t st) {
-  return dp::batch::launch_raw(bp->count, bp->max_n, bp->sms, bp->d_n, bp->d_offsets, bp->d_rec,
+  return dp::batch::launch_raw(bp->classes, bp->sms, bp->d_n, bp->d_offsets, bp->d_rec,
                                bp->d_order, bp->d_queue, d_base, d_ipiv, d_jpiv, d_info, bp->opt,
                                st);
 }
@@ -895,41 +1051,50 @@ namespace batch {
 // d_rec, d_order describe `count` matrices as in a dp_batch plan, d_queue is
 // kQueueBytes of 8-byte aligned scratch (the work counter, then the launch's
 // near-tie counters), cleared here before the launch.
-int launch_raw(int count, int max_n, int sms, const int* d_n, const long long* d_off,
+int launch_raw(const Classes& classes, int sms, const int* d_n, const long long* d_off,
                const long long* d_rec, const int* d_order, int* d_queue, double* base, int* ipiv,
                int* jpiv, int* info, const dp_batch_options& opt, cudaStream_t st) {
-  if (count <= 0) return DP_SUCCESS;
-  if (max_n < 1 || max_n > DP_BATCH_MAX_N || !valid_batch_options(&opt)) return DP_INVALID_ARGUMENT;
+  if (!valid_batch_options(&opt)) return DP_INVALID_ARGUMENT;
   Params p;
   p.base = base;
   p.offsets = d_off;
   p.ns = d_n;
   p.rec_offsets = d_rec;
-  p.order = d_order;
-  p.count = count;
-  p.queue = d_queue;
   p.ipiv = ipiv;
   p.jpiv = jpiv;
   p.info = info;
-  p.ties = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(d_queue) + 8);
+  p.ties = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(d_queue) + kTiesAt);
   p.threshold = opt.threshold;
   for (int i = 0; i < DP_BATCH_BUCKETS; ++i) p.nb_bucket[i] = opt.nb_bucket[i];
-  p.pr = panel_ld(max_n);
-  const size_t smem = dynamic_smem(max_n);
-  const int terms = dp::mixed_terms(opt.precision);
-  const void* fn = terms == 3   ? (const void*)batched_getrf_kernel<3>
-                   : terms == 2 ? (const void*)batched_getrf_kernel<2>
-                                : (const void*)batched_getrf_kernel<0>;
-  if (!dp::ensure_smem(fn, smem)) return DP_CUDA_FAILURE;
-  const int per_sm = dp::occupancy_once(fn, kThreads, smem);
-  if (per_sm < 1) return DP_CUDA_FAILURE;
-  const int grid = std::max(1, std::min(count, sms * per_sm));
   if (cudaMemsetAsync(d_queue, 0, kQueueBytes, st) != cudaSuccess) return DP_CUDA_FAILURE;
-  dp::note_launch();
-  void* args[] = {&p};
-  if (cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), args, smem, st) != cudaSuccess)
-    return DP_CUDA_FAILURE;
+  const int terms = dp::mixed_terms(opt.precision);
+  int first = 0, launched = 0;
+  for (int c = kClasses - 1; c >= 0; --c) {  // largest first, as the order is
+    if (classes.count[c] <= 0) continue;
+    p.order = d_order + first;
+    p.count = classes.count[c];
+    p.queue = d_queue + c;
+    const int top = classes.max_n[c];
+    const bool behind = launched > 0;
+    const int rc = c == 3   ? launch_class<Geo3>(p, top, sms, terms, behind, st)
+                   : c == 2 ? launch_class<Geo2>(p, top, sms, terms, behind, st)
+                   : c == 1 ? launch_class<Geo1>(p, top, sms, terms, behind, st)
+                            : launch_class<Geo0>(p, top, sms, terms, behind, st);
+    if (rc != DP_SUCCESS) return rc;
+    first += classes.count[c];
+    ++launched;
+  }
   return cudaGetLastError() == cudaSuccess ? DP_SUCCESS : DP_CUDA_FAILURE;
+}
+
+Classes classes_of(const int* ns, int count) {
+  Classes k;
+  for (int i = 0; i < count; ++i) {
+    const int c = class_of(ns[i]);
+    ++k.count[c];
+    k.max_n[c] = std::max(k.max_n[c], ns[i]);
+  }
+  return k;
 }
 
 }  // namespace batch
@@ -946,9 +1111,19 @@ int launch_panel_small(const PanelParams& pp, cudaStream_t st) {
   const int rows = pp.m - pp.begin, w = pp.end - pp.begin;
   if (rows < 1 || rows > batch::kMaxN || w < 1 || w > batch::kMaxNb) return kInvalidArgument;
   const size_t smem = (size_t)batch::panel_ld(rows) * batch::kMaxNb * sizeof(double);
-  if (!ensure_smem((const void*)batch::panel_small_kernel, smem)) return kCudaFailure;
-  note_launch();
-  batch::panel_small_kernel<<<1, batch::kThreads, smem, st>>>(pp);
+  // the fewest warps that hold the rows: a step's barrier and its merge of the
+  // warps' candidates get shorter
+  auto go = [&](auto geo) -> int {
+    using G = decltype(geo);
+    if (!ensure_smem((const void*)batch::panel_small_kernel<G>, smem)) return kCudaFailure;
+    note_launch();
+    batch::panel_small_kernel<G><<<1, G::T, smem, st>>>(pp);
+    return kOk;
+  };
+  const int rc = rows <= 128   ? go(batch::PanelGeo<128>{})
+                 : rows <= 256 ? go(batch::PanelGeo<256>{})
+                               : go(batch::PanelGeo<512>{});
+  if (rc != kOk) return rc;
   return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
 }
 
@@ -993,7 +1168,6 @@ int dp_batch_create(dp_batch** out, int count, const int* n, const long long* of
   bp->rec_offsets.resize(count);
   long long pos = 0, rec = 0;
   for (int i = 0; i < count; ++i) {
-    bp->max_n = std::max(bp->max_n, n[i]);
     if (offsets) {
       bp->offsets[i] = offsets[i];
       pos = std::max(pos, offsets[i] + (long long)n[i] * n[i]);
@@ -1004,6 +1178,7 @@ int dp_batch_create(dp_batch** out, int count, const int* n, const long long* of
     bp->rec_offsets[i] = rec;
     rec += n[i];
   }
+  bp->classes = dp::batch::classes_of(n, count);
   bp->total_elements = pos;
   bp->total_records = rec;
   if (cudaGetDevice(&bp->device) != cudaSuccess ||
@@ -1102,7 +1277,8 @@ int dp_batch_getrf_graph(dp_batch* bp, double* d_base, int* d_ipiv, int* d_jpiv,
     }
     std::copy(args, args + 4, bp->g_args);
   }
-  dp::note_launch();  // the graph holds one kernel (after the queue reset)
+  for (int c : bp->classes.count)  // the graph's kernels (after the queue reset)
+    if (c > 0) dp::note_launch();
   return cudaGraphLaunch(bp->exec, (cudaStream_t)stream) == cudaSuccess ? DP_SUCCESS
                                                                         : DP_CUDA_FAILURE;
 }
@@ -1112,7 +1288,7 @@ int dp_batch_last_report(dp_batch* bp, dp_getrf_report* out) {
   unsigned long long t[3] = {0, 0, 0};
   if (bp->count > 0 &&
       (cudaDeviceSynchronize() != cudaSuccess ||
-       cudaMemcpy(t, reinterpret_cast<char*>(bp->d_queue) + 8, sizeof(t),
+       cudaMemcpy(t, reinterpret_cast<char*>(bp->d_queue) + dp::batch::kTiesAt, sizeof(t),
                   cudaMemcpyDeviceToHost) != cudaSuccess))
     return DP_CUDA_FAILURE;
   std::memset(out, 0, sizeof(*out));

@@ -171,11 +171,15 @@ struct DecisionTally {
       }
     }
   }
-  __device__ __forceinline__ void flush(State* st) const {
-    if (checked) atomicAdd(&st->ties_checked, checked);
-    if (near) atomicAdd(&st->near_ties, near);
+  __device__ __forceinline__ void flush(unsigned long long* n_checked, unsigned long long* n_near,
+                                        unsigned long long* closeness) const {
+    if (checked) atomicAdd(n_checked, checked);
+    if (near) atomicAdd(n_near, near);
     if (c_sec > 0.0)
-      atomicMax(&st->closeness, (unsigned long long)__double_as_longlong(c_sec / c_best));
+      atomicMax(closeness, (unsigned long long)__double_as_longlong(c_sec / c_best));
+  }
+  __device__ __forceinline__ void flush(State* st) const {
+    flush(&st->ties_checked, &st->near_ties, &st->closeness);
   }
 };
 

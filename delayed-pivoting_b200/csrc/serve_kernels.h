@@ -8,12 +8,19 @@
 
 namespace dp {
 namespace batch {
-// Bytes of the scratch `d_queue` of launch_raw: the work counter and the
-// launch's near-tie counters (decisions checked, order-sensitive decisions,
-// largest runner-up / winner ratio as bits) at byte 8.
-constexpr size_t kQueueBytes = 32;
-// The batched factorisation on caller-managed device arrays (batched.cu).
-int launch_raw(int count, int max_n, int sms, const int* d_n, const long long* d_off,
+// Bytes of the scratch `d_queue` of launch_raw: a work counter per size class,
+// then the launch's near-tie counters (decisions checked, order-sensitive
+// decisions, largest runner-up / winner ratio as bits) at byte kTiesAt.
+constexpr int kClasses = 4;
+constexpr size_t kTiesAt = 16, kQueueBytes = 48;
+// Matrices and largest order of each size class.
+struct Classes {
+  int count[kClasses] = {}, max_n[kClasses] = {};
+};
+Classes classes_of(const int* ns, int count);
+// The batched factorisation on caller-managed device arrays (batched.cu);
+// d_order lists the matrices in decreasing order of size.
+int launch_raw(const Classes& classes, int sms, const int* d_n, const long long* d_off,
                const long long* d_rec, const int* d_order, int* d_queue, double* base, int* ipiv,
                int* jpiv, int* info, const dp_batch_options& opt, cudaStream_t st);
 }  // namespace batch

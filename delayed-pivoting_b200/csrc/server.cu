@@ -521,7 +521,6 @@ void dp_server::run_small_new(std::vector<Job>& jobs, cudaStream_t st) {
   g->off.resize(k);
   g->rec.resize(k);
   long long elems = 0, recs = 0;
-  int max_n = 1;
   for (int i = 0; i < k; ++i) {
     const int n = jobs[i].r.n;
     g->ns[i] = n;
@@ -529,7 +528,6 @@ void dp_server::run_small_new(std::vector<Job>& jobs, cudaStream_t st) {
     g->rec[i] = recs;
     elems += ((long long)n * n + 3) & ~3LL;
     recs += n;
-    max_n = std::max(max_n, n);
   }
   std::vector<int> order(k);
   for (int i = 0; i < k; ++i) order[i] = i;
@@ -598,7 +596,7 @@ void dp_server::run_small_new(std::vector<Job>& jobs, cudaStream_t st) {
     dp_batch_options bo;
     dp_batch_options_init(&bo);
     if (status == DP_SUCCESS)
-      status = dp::batch::launch_raw(k, max_n, sms, d_n, d_off, d_rec, d_order, d_queue, g->base,
+      status = dp::batch::launch_raw(dp::batch::classes_of(g->ns.data(), k), sms, d_n, d_off, d_rec, d_order, d_queue, g->base,
                                      g->ipiv, g->jpiv, g->info, bo, st);
     if (status == DP_SUCCESS)
       status = sv::launch_orders(d_n, d_rec, g->ipiv, g->jpiv, g->row, g->col, k, st);
