@@ -64,12 +64,12 @@ struct Cfg {
   static_assert(LDA_S % 16 == 4 && LDB_S % 16 == 4, "bank layout");
 };
 
+// The tile of C at (m0, n0).
 template <class C>
-__global__ void __launch_bounds__(C::THREADS, C::MINB)
-dgemm_minus_kernel(int M, int N, int K, const double* __restrict__ A, long long lda,
-                   const double* __restrict__ B, long long ldb, double* Cm, long long ldc,
-                   const int* gate, bool lower) {
-  if (gate && *gate >= 0) return;  // an enqueued panel sequence stopped before this update
+__device__ __forceinline__ void tile_minus(long long m0, long long n0, int M, int N, int K,
+                                           const double* __restrict__ A, long long lda,
+                                           const double* __restrict__ B, long long ldb, double* Cm,
+                                           long long ldc, bool lower) {
   extern __shared__ __align__(16) double gsm[];
   double* As = gsm;                         // [STAGES][BK][LDA_S]
   double* Bs = gsm + C::STAGES * C::A_STAGE;  // [STAGES][BN][LDB_S]
@@ -78,20 +78,6 @@ dgemm_minus_kernel(int M, int N, int K, const double* __restrict__ A, long long 
   const int lane = tid & 31, warp = tid >> 5;
   const int wm = warp / C::WARPS_N, wn = warp % C::WARPS_N;
   const int g = lane >> 2, t = lane & 3;
-  long long m0, n0;
-  if (lower) {
-    // Lower mode (M == N, C symmetric, its lower triangle only; BM == BN): a
-    // 1-D grid over the tiles (bi, bj) with bj <= bi, t = bi (bi + 1) / 2 + bj.
-    const long long t = blockIdx.x;
-    long long bi = (long long)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
-    while (bi * (bi + 1) / 2 > t) --bi;
-    m0 = bi * C::BM;
-    n0 = (t - bi * (bi + 1) / 2) * C::BN;
-  } else {
-    m0 = (long long)blockIdx.x * C::BM;
-    n0 = (long long)blockIdx.y * C::BN;
-  }
 
   // Prefetch this CTA's C tile into L2 (128-byte lines, in-bounds only).
   {
@@ -205,6 +191,43 @@ dgemm_minus_kernel(int M, int N, int K, const double* __restrict__ A, long long 
 }
 
 template <class C>
+__global__ void __launch_bounds__(C::THREADS, C::MINB)
+dgemm_minus_kernel(int M, int N, int K, const double* __restrict__ A, long long lda,
+                   const double* __restrict__ B, long long ldb, double* Cm, long long ldc,
+                   const int* gate, bool lower) {
+  if (gate && *gate >= 0) return;  // an enqueued panel sequence stopped before this update
+  long long m0, n0;
+  if (lower) {
+    // Lower mode (M == N, C symmetric, its lower triangle only; BM == BN): a
+    // 1-D grid over the tiles (bi, bj) with bj <= bi, t = bi (bi + 1) / 2 + bj.
+    const long long t = blockIdx.x;
+    long long bi = (long long)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
+    while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
+    while (bi * (bi + 1) / 2 > t) --bi;
+    m0 = bi * C::BM;
+    n0 = (t - bi * (bi + 1) / 2) * C::BN;
+  } else {
+    m0 = (long long)blockIdx.x * C::BM;
+    n0 = (long long)blockIdx.y * C::BN;
+  }
+  tile_minus<C>(m0, n0, M, N, K, A, lda, B, ldb, Cm, ldc, lower);
+}
+
+// The whole update by a grid of any size, and only when *run < 0.
+template <class C>
+__global__ void __launch_bounds__(C::THREADS, C::MINB)
+dgemm_minus_if_kernel(int M, int N, int K, const double* __restrict__ A, long long lda,
+                      const double* __restrict__ B, long long ldb, double* Cm, long long ldc,
+                      const int* run) {
+  if (*run >= 0) return;
+  const long long tm = (M + C::BM - 1) / C::BM, tiles = tm * ((N + C::BN - 1) / C::BN);
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+    tile_minus<C>(t % tm * C::BM, t / tm * C::BN, M, N, K, A, lda, B, ldb, Cm, ldc, false);
+    __syncthreads();  // the stages are free
+  }
+}
+
+template <class C>
 void launch(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
             double* Cm, long long ldc, cudaStream_t s, const int* gate, bool lower = false) {
   dp::ensure_smem((const void*)dgemm_minus_kernel<C>, C::SMEM);
@@ -281,6 +304,18 @@ void launch_gemm_minus(int M, int N, int K, const double* A, long long lda, cons
     gemm::launch<gemm::SmallK32>(M, N, K, A, lda, B, ldb, C, ldc, s, gate);
   else
     gemm::launch<gemm::Small4>(M, N, K, A, lda, B, ldb, C, ldc, s, gate);
+}
+
+// C -= A * B when *run < 0 (read when the kernel starts), nothing otherwise:
+// few CTAs over all tiles, since this launch nearly always has nothing to do.
+void launch_gemm_minus_if(int M, int N, int K, const double* A, long long lda, const double* B,
+                          long long ldb, double* C, long long ldc, cudaStream_t s, const int* run) {
+  if (M <= 0 || N <= 0 || K <= 0) return;
+  using Tile = gemm::Small4;
+  ensure_smem((const void*)gemm::dgemm_minus_if_kernel<Tile>, Tile::SMEM);
+  note_launch();
+  gemm::dgemm_minus_if_kernel<Tile><<<4 * sm_count(), Tile::THREADS, Tile::SMEM, s>>>(
+      M, N, K, A, lda, B, ldb, C, ldc, run);
 }
 
 // Lower triangle of the symmetric N x N block C -= A(N x K) * B(K x N), the

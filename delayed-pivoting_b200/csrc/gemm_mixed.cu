@@ -33,6 +33,7 @@
 
 #include "dp_device.cuh"
 #include "dp_kernels.h"
+#include "umma.cuh"
 
 namespace dp {
 
@@ -98,60 +99,7 @@ __global__ void split_b_kernel(const double* __restrict__ B, long long ldb, int 
   }
 }
 
-// ------------------------------------------------------ PTX wrappers ----
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-// Bounded wait for the phase with the given parity; false on timeout.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const uint32_t addr = smem_u32(bar);
-  const unsigned long long t0 = globaltimer_ns();
-  for (unsigned it = 0;; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((it & 255u) == 255u && globaltimer_ns() - t0 > kSpinLimitNs) return false;
-  }
-}
-
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, uint64_t* bar, int x,
-                                            int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major, 128-byte-swizzled operand
-// tile (8-row x 128-byte swizzle atoms, atoms 1024 bytes apart).
-__device__ __forceinline__ uint64_t umma_desc_k_sw128(const void* tile) {
-  const uint64_t addr = smem_u32(tile);
-  uint64_t d = 0;
-  d |= (addr >> 4) & 0x3FFFull;          // start address (16-byte units)
-  d |= 1ull << 16;                        // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;       // stride byte offset: next 8-row group
-  d |= 1ull << 46;                        // descriptor version (sm_100)
-  d |= 2ull << 61;                        // layout: 128-byte swizzle
-  return d;
-}
+using namespace umma;
 
 // kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, both
 // K-major, M = 128, N = 128.
@@ -168,23 +116,6 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15},"
-      " [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // -------------------------------------------------------------- GEMM ----
@@ -215,10 +146,6 @@ constexpr int kThreadsP = 64 + 32 * kEpiWarps;  // 576
 constexpr int kEpiCols = BN / (kEpiWarps / 4);  // 32 columns per epilogue thread
 constexpr unsigned kTmemColsP = 2 * BN;         // double-buffered accumulator
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 template <int TERMS>
 __global__ void __launch_bounds__(kThreadsP, 1)
 gemm_bf16x3_kernel(const __grid_constant__ Maps tm, int M, int N, int kchunks, double* C,
@@ -231,7 +158,8 @@ gemm_bf16x3_kernel(const __grid_constant__ Maps tm, int M, int N, int kchunks, d
   __shared__ int failed;
   unsigned char* smem =
       reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(~0u, tid >> 5, 0);  // (uniform)
   const int tiles_m = (M + BM - 1) / BM;
   const int tiles = tiles_m * ((N + BN - 1) / BN);
 
@@ -268,7 +196,7 @@ gemm_bf16x3_kernel(const __grid_constant__ Maps tm, int M, int N, int kchunks, d
   };
 
   if (warp == 0) {
-    if (lane == 0) {  // TMA producer
+    if (elect_one()) {  // TMA producer
       int g = 0;      // chunk counter over this CTA's tiles
       for (int t = blockIdx.x; t < tiles && !*vfailed; t += gridDim.x) {
         const int m0 = (t % tiles_m) * BM, n0 = (t / tiles_m) * BN;
@@ -290,7 +218,7 @@ gemm_bf16x3_kernel(const __grid_constant__ Maps tm, int M, int N, int kchunks, d
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // MMA issuer
+    if (elect_one()) {  // MMA issuer
       const uint32_t idesc = idesc_bf16_f32(BM, BN);
       int g = 0, it = 0;
       bool ok = true;
@@ -389,36 +317,10 @@ gemm_bf16x3_kernel(const __grid_constant__ Maps tm, int M, int N, int kchunks, d
 }
 
 // ------------------------------------------------------ host helpers ----
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
 // 2-D BF16 tensor [rows][kp] (kp contiguous), box 64 x 128, 128-byte swizzle.
 bool make_map(CUtensorMap* tm, void* base, int rows, int kp) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)kp, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)kp * 2};
-  cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)BM};
-  cuuint32_t estr[2] = {1, 1};
-  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  return encode_map(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, kp, rows, (cuuint64_t)kp * 2, BK, BM,
+                    CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 }  // namespace mixed

@@ -130,6 +130,7 @@ struct Workspace {
   int* swap_extra = nullptr;
   Cand* cands = nullptr;
   void* mixed = nullptr;   // BF16 operand scratch of the tensor-core update (mixed precision)
+  void* i8 = nullptr;      // digits of the integer-core update (i8_update), nullptr: not used
   void* mixed1 = nullptr;  // the same for the next outer block's update on the panel stream
   // Look-ahead: swap lists of the panels of an outer block, kept until the
   // block completes (two buffers, alternating between consecutive blocks;
@@ -171,7 +172,7 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 // Lays the workspace out from `base` (nullptr: only computes the size).
 size_t layout_workspace(Workspace& ws, char* base, int pivots, int max_ctas, int w_max,
                         size_t mixed_bytes, int defer_cap = 0, size_t mixed1_bytes = 0,
-                        const InvPlan& inv = InvPlan{}) {
+                        const InvPlan& inv = InvPlan{}, size_t i8_mem = 0) {
   size_t off = 0;
   auto take = [&](size_t bytes) {
     const size_t at = off;
@@ -199,6 +200,7 @@ size_t layout_workspace(Workspace& ws, char* base, int pivots, int max_ctas, int
   ws.scratch = base ? base + off : nullptr;
   ws.mixed = mixed_bytes ? reinterpret_cast<void*>(take(mixed_bytes)) : nullptr;
   ws.mixed1 = mixed1_bytes ? reinterpret_cast<void*>(take(mixed1_bytes)) : nullptr;
+  ws.i8 = i8_mem ? reinterpret_cast<void*>(take(i8_mem)) : nullptr;
   ws.tinv_ld = inv.ld;
   if (inv.ld > 0) {
     const size_t ld = (size_t)inv.ld;
@@ -396,11 +398,28 @@ struct BlockInv {
   double* copy = nullptr;  // ldt x (columns) doubles
 };
 
+// The rank-W update of a finished block on the integer tensor cores: A's digits
+// are taken in the first update_columns call that has it, and serve the calls
+// after it on the same stream (`ready`).
+struct I8Block {
+  I8Update u;
+  bool ready = false;
+};
+constexpr int kI8ScaleCols = 64;  // columns of U12 that balance the W terms
+
+// Where it is used: below about 2000 x 2000 the splits and the tensor path's
+// start eat the gain (K = 256, FP64 path / this, us: 1024 x 1024 32 / 37,
+// 2048 x 2048 92 / 82, 4096 x 4096 329 / 219, 16384 x 16384 4773 / 2469), below
+// K = 128 the traffic of C does (8192 x 8192: K = 64 369 / 374, 128 656 / 455).
+bool use_i8(long long rows, long long cols, int W) {
+  return W >= 128 && W <= i8_max_k() && rows >= 512 && cols >= 512 && rows * cols >= 2000LL * 2000;
+}
+
 // `solved`: the block rows already hold U12 (the panel's laswp solved them).
 int update_columns(double* a, long long lda, int m, int s0, int W, int r_gemm, int c0, int n_end,
                    cudaStream_t st, Recorder& rec, void* mixed_ws = nullptr,
                    int* status = nullptr, int terms = 2, const int* gate = nullptr,
-                   const BlockInv* bi = nullptr, bool solved = false) {
+                   const BlockInv* bi = nullptr, bool solved = false, I8Block* i8 = nullptr) {
   const int nc = n_end - c0;
   if (W <= 0 || nc <= 0) return kOk;
   if (solved) {
@@ -426,6 +445,20 @@ int update_columns(double* a, long long lda, int m, int s0, int W, int r_gemm, i
     return e;
   }
   rec.begin(DP_KFAM_GEMM);
+  if (i8) {
+    const double *A = a + idx(r_gemm, s0, lda), *U = a + idx(s0, c0, lda);
+    int e = kOk, launches = 3;
+    if (!i8->ready) {
+      e = launch_i8_split_a(i8->u, M, W, A, lda, U, lda, std::min(kI8ScaleCols, nc), st);
+      i8->ready = true;
+      launches += 2;
+    }
+    if (e == kOk)
+      e = launch_gemm_minus_i8(i8->u, M, nc, W, A, lda, U, lda, a + idx(r_gemm, c0, lda), lda,
+                               status, st);
+    rec.end(fl, by, launches);
+    return e;
+  }
   launch_gemm_minus(M, nc, W, a + idx(r_gemm, s0, lda), lda, a + idx(s0, c0, lda), lda,
                     a + idx(r_gemm, c0, lda), lda, st, gate);
   rec.end(fl, by, 1);
@@ -577,6 +610,16 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
     on2 = BlockInv{T, ws.tinv_ld, ws.tcopy2};
   };
   BlockInv inv1, inv2;
+  // the integer-core update of block [B, .) of width W on rows r.. and columns
+  // c.. (FP64 precision only; the next block's columns always take the FP64
+  // kernel, so that both schedules do the same arithmetic)
+  auto integer_update = [&](int r, int c, int W, I8Block& blk) -> I8Block* {
+    if (!ws.i8 || terms || !use_i8(m - r, n - c, W)) return nullptr;
+    blk.u = i8_update(ws.i8, m, n);
+    blk.ready = false;
+    return &blk;
+  };
+  I8Block i8blk;
   while (B < pivots) {
     const int E = std::min(pivots, B + NB);
     int* blk = la ? ws.defer_blk + (size_t)half * ws.defer_cap : ws.swap_block;
@@ -739,8 +782,14 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
       // right of the outer block: the O(n^3) update
       inv1 = inv2 = BlockInv{};
       if (E < n) block_inverse(B, E - B, 0, inv1, inv2);
-      if (int err = update_columns(a, lda, m, B, E - B, E, E, n, st, rec, mixed_ws,
-                                   &ws.state->status, terms, nullptr, &inv2))
+      const int NE = std::min(pivots, E + NB);
+      I8Block* i8 = integer_update(E, NE, E - B, i8blk);
+      if (i8)  // the next block's columns first, as with look-ahead
+        if (int err = update_columns(a, lda, m, B, E - B, E, E, NE, st, rec, nullptr,
+                                     &ws.state->status, terms, nullptr, &inv2))
+          return err;
+      if (int err = update_columns(a, lda, m, B, E - B, E, i8 ? NE : E, n, st, rec, mixed_ws,
+                                   &ws.state->status, terms, nullptr, &inv2, false, i8))
         return err;
       DP_CHECK_CUDA(cudaGetLastError());
       B = E;
@@ -788,15 +837,16 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
         return err;
       DP_CHECK_CUDA(cudaEventRecord(sc.ldone, sc.s3));
       pending = false;
+      I8Block* i8 = integer_update(E, NE, E - B, i8blk);
       if (NNE > NE) {
         if (int err = update_columns(a, lda, m, B, E - B, E, NE, NNE, sc.s2, *sc.r2, mixed_ws,
-                                     ws.aux_status, terms, nullptr, &inv2))
+                                     ws.aux_status, terms, nullptr, &inv2, false, i8))
           return err;
         DP_CHECK_CUDA(cudaEventRecord(sc.next, sc.s2));
         pending = true;
       }
       if (int err = update_columns(a, lda, m, B, E - B, E, std::max(NE, NNE), n, sc.s2, *sc.r2,
-                                   mixed_ws, ws.aux_status, terms, nullptr, &inv2))
+                                   mixed_ws, ws.aux_status, terms, nullptr, &inv2, false, i8))
         return err;
       DP_CHECK_CUDA(cudaGetLastError());
       half ^= 1;
@@ -820,8 +870,8 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
     inv1 = inv2 = BlockInv{};
     if (E < n) block_inverse(B, k - B, half, inv1, inv2);
     if (int err = update_columns(a, lda, m, B, k - B, k, E, n, st, rec, mixed_ws,
-                                 &ws.state->status, terms, nullptr,
-                                 &inv2))  // right of the outer block
+                                 &ws.state->status, terms, nullptr, &inv2, false,
+                                 integer_update(k, E, k - B, i8blk)))  // right of the outer block
       return err;
     rec.begin(DP_KFAM_SEARCH);
     if (o.policy == DP_POLICY_NONZERO_COLUMN)
@@ -961,15 +1011,20 @@ int getrf_device(int m, int n, double* d_a, int lda, int* ipiv, int* jpiv, int* 
     ip.copy1_cols = lanes ? NB : 0;
     ip.copy2_cols = n;
   }
+  // the first block's update is the largest
+  const size_t i8_mem = !mixed_terms(o.precision) && use_i8(m - (long long)NB, n - 2LL * NB, NB)
+                            ? i8_bytes(m, n)
+                            : 0;
   const size_t bytes = layout_workspace(ws, nullptr, pivots, di.sms, w_max, mixed_bytes,
-                                        defer_cap, mixed1_bytes, ip);
+                                        defer_cap, mixed1_bytes, ip, i8_mem);
   char* base = nullptr;
   if (dp::workspace_alloc(reinterpret_cast<void**>(&base), bytes, st) != cudaSuccess) {
     cudaGetLastError();
     *info = -1;
     return kAllocationFailed;
   }
-  layout_workspace(ws, base, pivots, di.sms, w_max, mixed_bytes, defer_cap, mixed1_bytes, ip);
+  layout_workspace(ws, base, pivots, di.sms, w_max, mixed_bytes, defer_cap, mixed1_bytes, ip,
+                   i8_mem);
   int status = kOk;
   // the scratch regions (at the end) are fully written before use; clear the rest
   const size_t clear = (size_t)(ws.scratch - base);
