@@ -42,6 +42,7 @@ size_t panel_cluster_smem_bytes(int w, int rows_per_cta);
 // (nullptr beyond the limit) and its dynamic shared memory.
 int panel_reg_max_rows();
 const void* panel_reg_kernel_for(int rows_per_cta);
+int panel_reg_threads(int rows_per_cta);
 size_t panel_reg_smem_bytes(int w, int rows_per_cta);
 int panel_cluster_threads();
 constexpr int kPanelThreadsHost = 256;

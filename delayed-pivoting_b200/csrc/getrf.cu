@@ -695,7 +695,7 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cfg.gridDim = dim3(G);
-        cfg.blockDim = dim3(panel_cluster_threads());
+        cfg.blockDim = dim3(use_reg ? panel_reg_threads(R) : panel_cluster_threads());
         cfg.dynamicSmemBytes =
             use_reg ? panel_reg_smem_bytes(w, R) : panel_cluster_smem_bytes(w, R);
         cfg.stream = st;

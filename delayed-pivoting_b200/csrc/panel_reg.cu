@@ -1,5 +1,5 @@
 // Panel factorisation on one thread-block cluster with the sub-panel in
-// registers (panels of up to 512 rows per CTA).
+// registers (panels of up to 1024 rows per CTA).
 //
 // Same contract and semantics as panel_cluster_kernel
 // (delayed_lu/delayed_dgetrf.cpp:164-240: column partial-pivot search with
@@ -22,10 +22,11 @@
 //     owning CTAs' shared memory (phase A), a second cluster barrier, then
 //     writes them in place (phase B) and applies the rank-8 update of the
 //     columns right of the sub-panel.
-// Push buffers are indexed by step parity: a slot written at step s + 2 is
-// written after the barrier of step s + 1, which every reader of step s
-// passes only after finishing step s.  No spin-waits: the only waits are the
-// hardware barriers.
+// Push buffers are indexed by step parity: a slot is written again at step s +
+// 2, which every CTA reaches only through the barrier of step s + 1, passed by
+// every reader of step s.  The waits for a step's slots are bounded; a thread
+// whose wait runs out records the status and leaves with its whole CTA at the
+// next CTA barrier.
 #include <cooperative_groups.h>
 
 #include "dp_device.cuh"
@@ -44,8 +45,7 @@ using panel::warp_best;
 using panel::warp_lb;
 using panel::warp_max_pos;
 
-constexpr int kT = 256;      // threads
-constexpr int kW = kT / 32;  // warps
+constexpr int kMaxW = 16;    // most warps of a CTA
 constexpr int kS = 8;        // sub-panel width
 constexpr int kMaxC = 16;    // largest cluster
 
@@ -80,11 +80,12 @@ struct Layout {
   double* sm;     // [w][RP] the panel slice
   Slot* slots;    // [2][kMaxC] candidates, by step parity and CTA rank
   Slot* kslot;    // [2] row k, by step parity
-  Slot* stage;    // [kW] per-warp candidates, then [1] row k
+  Slot* stage;    // [kMaxW] per-warp candidates, then [1] row k
   double* psave;  // [kS][W1] the sub-panel's pivot rows
   double* tmp;    // [2 kS][W1] pulled content of moved rows (by map entry)
   int* orig;      // [R] source row of each local row
   int* plist;     // [kS][2] (k, pivot row) of the sub-panel's steps
+  int* pivs;      // [w] pivot rows (rank 0)
   int* own;       // [1 + 3 * 2 kS]: count, then (local row, source owner, source
                   // local row) of the moved rows this CTA owns
   int* ksrc;      // [2 kS]: (owner, local row) of the content of each step's row k
@@ -104,11 +105,12 @@ __host__ __device__ inline size_t reg_layout(unsigned char* base, int w, int R, 
   unsigned char* sm = take(sizeof(double) * (size_t)w * rp);
   unsigned char* slots = take(sizeof(Slot) * 2 * kMaxC);
   unsigned char* kslot = take(sizeof(Slot) * 2);
-  unsigned char* stage = take(sizeof(Slot) * (kW + 1));
+  unsigned char* stage = take(sizeof(Slot) * (kMaxW + 1));
   unsigned char* psave = take(sizeof(double) * kS * w1);
   unsigned char* tmp = take(sizeof(double) * 2 * kS * w1);  // row q: map entry q
   unsigned char* orig = take(sizeof(int) * (size_t)R);
   unsigned char* plist = take(sizeof(int) * 2 * kS);
+  unsigned char* pivs = take(sizeof(int) * (size_t)w);
   unsigned char* own = take(sizeof(int) * (1 + 6 * kS));
   unsigned char* ksrc = take(sizeof(int) * 2 * kS);
   unsigned char* xbar = take(sizeof(unsigned long long) * 2);
@@ -121,6 +123,7 @@ __host__ __device__ inline size_t reg_layout(unsigned char* base, int w, int R, 
     L->tmp = reinterpret_cast<double*>(tmp);
     L->orig = reinterpret_cast<int*>(orig);
     L->plist = reinterpret_cast<int*>(plist);
+    L->pivs = reinterpret_cast<int*>(pivs);
     L->own = reinterpret_cast<int*>(own);
     L->ksrc = reinterpret_cast<int*>(ksrc);
     L->xbar = reinterpret_cast<unsigned long long*>(xbar);
@@ -130,8 +133,9 @@ __host__ __device__ inline size_t reg_layout(unsigned char* base, int w, int R, 
 
 }  // namespace
 
-template <int RPT>
+template <int kT, int RPT>
 __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
+  constexpr int kW = kT / 32;
   // Every CTA reads the same word before any barrier or state write (a stop
   // is recorded only by an earlier kernel), so all of them leave together.
   if (p.gated && p.state->stop_k >= 0) return;
@@ -173,17 +177,23 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
   // peer reads the one or writes to the other
   cluster.sync();
 
-  // candidate of column 0
   LocalBest mine{0.0, -1, 0, 0.0};
   double mine_x = 0.0;  // signed entry of the candidate
-#pragma unroll
-  for (int i = 0; i < RPT; ++i) {
-    const int r = tid + i * kT;
-    if (r < rows_here) offer_x(mine, mine_x, sm[r], r);
-  }
 
-  DecisionTally tally;  // rank 0, thread 0 records the decisions
-  bool stopped = false, timed_out = false;
+  // Near-tie record (rank 0, warp 0, recorded by its lane 0): a decision's
+  // runner-up is reduced and tallied while the next exchange is awaited
+  DecisionTally tally;
+  long long t_k = -1;  // the decision to record, -1 when none
+  double t_best = 0.0, t_lane = 0.0;
+  auto record = [&] {
+    if (rank == 0 && warp == 0 && t_k >= 0) {
+      const double second = warp_max_pos(t_lane);
+      if (lane == 0) tally.note(t_k, t_best, second);
+      t_k = -1;
+    }
+  };
+  bool stopped = false, timed_out = false, late = false;
+  int done = 0;  // steps executed
   bool pending = false;  // a cluster_arrive() awaits its cluster_wait()
   for (int base = 0; base < w && !stopped; base += kS) {
     const int send = min(base + kS, w);
@@ -194,6 +204,13 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
 #pragma unroll
       for (int t = 0; t < kS; ++t)
         x[i][t] = (r < rows_here && base + t < w) ? sm[(base + t) * RP + r] : 0.0;
+    }
+    // the candidate of the sub-panel's first column
+    mine = LocalBest{0.0, -1, 0, 0.0};
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = tid + i * kT;
+      if (r < rows_here && row0 + r >= (long long)p.begin + base) offer_x(mine, mine_x, x[i][0], r);
     }
     int kd = send - base;  // steps executed in this sub-panel
 
@@ -243,7 +260,7 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
         st.orig = -1;
       }
       if (own_k && tid == kl % kT) {
-        Slot& st = S.stage[kW];
+        Slot& st = S.stage[kMaxW];
         const int ki = kl / kT;
 #pragma unroll
         for (int i = 0; i < RPT; ++i)
@@ -254,26 +271,30 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
         st.orig = orig[kl];
         st.row = (int)k;
       }
-      __syncthreads();
-      // 2. the CTA's winner among the warps, pushed to every CTA
-      {
+      // (a wait of the step before that ran out ends every thread here)
+      if (__syncthreads_or(late)) {
+        timed_out = stopped = true;
+        kd = 0;
+        break;
+      }
+      // 2. the CTA's winner among the warps, pushed to every CTA (warp 0 alone:
+      //    the other warps leave the SM's reduction unit to it)
+      if (warp == 0) {
         const Slot* cs = S.stage + (lane & (kW - 1));
         const bool have = lane < kW && cs->row >= 0;
+        const double v = cs->val, sc = cs->sec;
         double bv;
         int brow;
-        warp_best(have ? cs->val : 0.0, have ? cs->row : 0x7fffffff, bv, brow);
-        const double bsec = warp_max_pos(
-            lane < kW ? ((have && cs->row == brow) ? cs->sec : (have ? cs->val : cs->sec)) : 0.0);
-        const int wsel = __ffs(__ballot_sync(0xffffffffu, have && cs->row == brow)) - 1;
-        if (warp == 0 && lane < C) {
+        warp_best(have ? v : 0.0, have ? cs->row : 0x7fffffff, bv, brow);
+        const bool won = have && cs->row == brow;
+        const int wsel = max(0, __ffs(__ballot_sync(0xffffffffu, won)) - 1);
+        const double bsec = warp_max_pos(lane < kW ? (won || !have ? sc : v) : 0.0);
+        if (lane < C) {
           uint4 c[kSlotChunks];
-          const uint4* src = reinterpret_cast<const uint4*>(S.stage + (wsel >= 0 ? wsel : 0));
+          const uint4* src = reinterpret_cast<const uint4*>(S.stage + wsel);
 #pragma unroll
           for (int i = 0; i < kSlotChunks; ++i) c[i] = src[i];
-          if (wsel < 0) {  // no candidate: magnitude 0, row -1, reciprocal 0
-            c[0].x = c[0].y = 0u;
-            c[1] = make_uint4(0u, 0u, 0xffffffffu, 0xffffffffu);
-          }
+          // (a warp without a candidate staged magnitude 0, row -1, reciprocal 0)
           const unsigned long long sb = (unsigned long long)__double_as_longlong(bsec);
           c[0].z = (unsigned)sb;
           c[0].w = (unsigned)(sb >> 32);
@@ -282,52 +303,70 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
 #pragma unroll
           for (int i = 0; i < kSlotChunks; ++i) panel::st_async16(dst + 16u * i, c[i], bar);
         }
-        if (warp == 1 && own_k && lane < C) {
-          const uint4* src = reinterpret_cast<const uint4*>(S.stage + kW);
-          const unsigned dst = panel::peer_addr(panel::smem_addr(S.kslot + par), lane);
-          const unsigned bar = panel::peer_addr(xb, lane);
+      } else if (warp == 1 && own_k && lane < C) {
+        const uint4* src = reinterpret_cast<const uint4*>(S.stage + kMaxW);
+        const unsigned dst = panel::peer_addr(panel::smem_addr(S.kslot + par), lane);
+        const unsigned bar = panel::peer_addr(xb, lane);
 #pragma unroll
-          for (int i = 0; i < kSlotChunks; ++i) panel::st_async16(dst + 16u * i, src[i], bar);
-        }
+        for (int i = 0; i < kSlotChunks; ++i) panel::st_async16(dst + 16u * i, src[i], bar);
       }
+      record();
       // every CTA's slot and row k's slice have arrived (use s >> 1 of this
-      // parity's barrier)
-      if (__syncthreads_or(!panel::xbar_wait(xb, (unsigned)(s >> 1) & 1u))) {
-        if (tid == 0) p.state->status = kDeviceTimeout;
-        timed_out = stopped = true;
-        kd = 0;
-        break;
+      // parity's barrier).  No CTA barrier here: the stage is read before its
+      // CTA's slot is pushed, and a slot buffer is written again only after
+      // every thread has passed the next step's barrier.  A wait that runs out
+      // goes on with stale slots (used for values and in-range compares only)
+      // to the next barrier, where all threads leave together
+      if (!panel::xbar_wait(xb, (unsigned)(s >> 1) & 1u)) {
+        late = true;
+        p.state->status = kDeviceTimeout;
       }
 
-      // 3. same decision everywhere
+      // 3. same decision everywhere (rows carry their slot in the low bits: the
+      //    smallest key is the smallest row, and names the winner's slot)
       int wslot = -1;
-      double wval = 0.0, wsec = 0.0;
+      double wval = 0.0;
       {
         const Slot* cs = S.slots + par * kMaxC + (lane < C ? lane : 0);
         const bool have = lane < C && cs->row >= 0;
-        double bv;
-        int brow;
-        warp_best(have ? cs->val : 0.0, have ? cs->row : 0x7fffffff, bv, brow);
-        wsec = warp_max_pos(lane < C ? ((have && cs->row == brow) ? cs->sec
-                                                                 : (have ? cs->val : cs->sec))
-                                     : 0.0);
-        if (brow != 0x7fffffff) {
-          wslot = __ffs(__ballot_sync(0xffffffffu, have && cs->row == brow)) - 1;
-          wval = bv;
+        const double v = lane < C ? cs->val : 0.0;
+        const unsigned long long u = (unsigned long long)__double_as_longlong(have ? v : 0.0);
+        const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
+        const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+        const bool top = have && hi == mhi && lo == mlo;
+        const unsigned key = __reduce_min_sync(
+            0xffffffffu, top ? ((unsigned)(cs->row - p.begin) << 4) | (unsigned)lane : 0xffffffffu);
+        if (key != 0xffffffffu) {
+          wslot = (int)(key & 15u);
+          wval = __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
+        }
+        if (rank == 0 && warp == 0 && !positioned) {
+          t_k = k;
+          t_best = wval;
+          t_lane = lane < C ? (lane == wslot || !have ? cs->sec : v) : 0.0;
         }
       }
-      if (rank == 0 && tid == 0 && !positioned) tally.note(k, wval, wsec);
       const bool stop = !positioned && !(wslot >= 0 && wval > p.threshold);
       if (stop) {
-        if (rank == 0 && tid == 0) p.state->stop_k = (int)k;
-        kd = j;
+        // (stale slots may stop some threads only: they meet the others, who
+        // are at the next step's barrier, and all leave)
         stopped = true;
+        kd = j;
+        if (__syncthreads_or(late)) {
+          timed_out = true;
+          kd = 0;
+        } else if (rank == 0 && tid == 0) {
+          p.state->stop_k = (int)k;
+        }
         break;
       }
       const Slot& ws = S.slots[par * kMaxC + wslot];
       const long long prow = ws.row;
-      if (rank == 0 && tid == 0 && !positioned) p.ipiv[k] = (int)prow;
       if (tid == 0) {
+        // (to memory at the end: a store on its way would hold up every release
+        // of the cluster barrier, about 1500 cycles a sub-panel)
+        S.pivs[s] = (int)prow;
         S.plist[2 * j] = (int)k;
         S.plist[2 * j + 1] = (int)prow;
       }
@@ -377,6 +416,7 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
     }
 
     // ---- end of the sub-panel: kd steps executed at [base, base + kd) ----
+    done = base + kd;
     if (kd == 0) break;  // stopped at its first step: nothing moved
     // a. the register slices back to shared memory
 #pragma unroll
@@ -396,24 +436,25 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
     //    owns (a pivot row that is also a later step's row k once), each with
     //    its source's owner and local row
     if (warp == 0) {
+      __syncwarp();  // the steps' list is lane 0's
       const bool on = lane < 2 * kd;
-      int x = on ? S.plist[lane < kd ? 2 * lane : 2 * (lane - kd) + 1] : 0;
+      int2 sw[kS];  // (k, pivot row) of the steps
+#pragma unroll
+      for (int t = 0; t < kS; ++t)
+        sw[t] = t < kd ? *reinterpret_cast<const int2*>(S.plist + 2 * t) : make_int2(-1, -1);
+      int x = on ? S.plist[lane < kd ? 2 * lane : 2 * (lane - kd) + 1] : -2 - lane;
       const int pos = x;
-      for (int t = kd - 1; t >= 0 && on; --t) {
-        const int a = S.plist[2 * t], b = S.plist[2 * t + 1];
-        x = x == a ? b : (x == b ? a : x);
-      }
+#pragma unroll
+      for (int t = kS - 1; t >= 0; --t) x = x == sw[t].x ? sw[t].y : (x == sw[t].y ? sw[t].x : x);
       const int so = on ? (int)((x - p.begin) / R) : 0;
       const int sl = on ? (int)(x - p.begin - (long long)so * R) : 0;
       if (lane < kd) {
         S.ksrc[2 * lane] = so;
         S.ksrc[2 * lane + 1] = sl;
       }
-      bool keep = on && x != pos && pos >= row0 && pos < row0 + rows_here;
-      for (int q = 0; q < 2 * kS; ++q) {  // first occurrence of each position
-        const int other = __shfl_sync(0xffffffffu, pos, q);
-        if (q < lane && q < 2 * kd && other == pos) keep = false;
-      }
+      // the first occurrence of each position
+      const bool first = __ffs(__match_any_sync(0xffffffffu, pos)) - 1 == lane;
+      const bool keep = on && first && x != pos && pos >= row0 && pos < row0 + rows_here;
       const unsigned bal = __ballot_sync(0xffffffffu, keep);
       if (keep) {
         const int at = __popc(bal & ((1u << lane) - 1u));
@@ -423,92 +464,72 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
       }
       if (lane == 0) S.own[0] = __popc(bal);
     }
-    __syncthreads();
+    if (__syncthreads_or(late)) {
+      timed_out = stopped = true;
+      break;
+    }
     const int nown = S.own[0];
     // the owners' writes of the previous sub-panel end are visible
     if (pending) {
       panel::cluster_wait();
       pending = false;
     }
-    const int ncol_out = base + (w - send);  // columns outside the sub-panel
-    auto out_col = [&](int c) { return c < base ? c : send + (c - base); };
     // c. phase A: the moved rows of this CTA (into tmp, row q for own entry
     //    q) and the pivot rows' columns right of the sub-panel (into psave),
-    //    read from their owners' shared memory; every (row, column) element
-    //    is an independent load, four per thread in flight
-    {
-      const int na = nown * ncol_out;
-      for (int e0 = tid; e0 < na; e0 += 4 * kT) {
+    //    read from their owners' shared memory: a thread takes a column and
+    //    every (kT / 64)-th row, four independent loads in flight
+    constexpr int kGrp = kT / 64;
+    const int cl = tid & 63, grp = tid >> 6;
+    const int nfetch = nown + (send < w ? kd : 0);
+    for (int c = cl; c < w; c += 64) {
+      if (c >= base && c < send) continue;
+      for (int q0 = grp; q0 < nfetch; q0 += 4 * kGrp) {
         double v[4];
-        int at[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int e = e0 + u * kT;
-          at[u] = -1;
-          if (e < na) {
-            const int q = e / ncol_out, c = e - q * ncol_out;
-            const double* src = cluster.map_shared_rank(sm, S.own[2 + 3 * q]);
-            v[u] = src[out_col(c) * RP + S.own[3 + 3 * q]];
-            at[u] = q * W1 + c;
-          }
+          const int q = q0 + u * kGrp;
+          if (q >= nfetch || (q >= nown && c < send)) continue;
+          const int* at = q < nown ? S.own + 2 + 3 * q : S.ksrc + 2 * (q - nown);
+          v[u] = cluster.map_shared_rank(sm, at[0])[c * RP + at[1]];
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (at[u] >= 0) S.tmp[at[u]] = v[u];
-      }
-    }
-    if (send < w) {
-      const int nr = w - send, np = kd * nr;
-      for (int e0 = tid; e0 < np; e0 += 4 * kT) {
-        double v[4];
-        int at[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int e = e0 + u * kT;
-          at[u] = -1;
-          if (e < np) {
-            const int t = e / nr, c = send + (e - t * nr);
-            const double* src = cluster.map_shared_rank(sm, S.ksrc[2 * t]);
-            v[u] = src[c * RP + S.ksrc[2 * t + 1]];
-            at[u] = t * W1 + c;
-          }
+          const int q = q0 + u * kGrp;
+          if (q >= nfetch || (q >= nown && c < send)) continue;
+          (q < nown ? S.tmp + q * W1 : S.psave + (q - nown) * W1)[c] = v[u];
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (at[u] >= 0) S.psave[at[u]] = v[u];
       }
     }
     cluster.sync();  // every CTA has read what it needs before anyone overwrites
     // d. phase B: moved rows take their sources' content
-    for (int e = tid; e < nown * ncol_out; e += kT) {
-      const int q = e / ncol_out, c = e - q * ncol_out;
-      sm[out_col(c) * RP + S.own[1 + 3 * q]] = S.tmp[q * W1 + c];
-    }
+    for (int c = cl; c < w; c += 64)
+      if (c < base || c >= send)
+        for (int q = grp; q < nown; q += kGrp) sm[c * RP + S.own[1 + 3 * q]] = S.tmp[q * W1 + c];
     if (send >= w) break;  // no columns right of the sub-panel
     __syncthreads();       // psave and the moved rows complete
-    // e. U12 = L11^{-1} A12 of the sub-panel, one column per thread
+    // e. U12 = L11^{-1} A12 of the sub-panel, one column per thread, a step's
+    //    multiples subtracted from all later rows before the next step (the
+    //    dependent chain is kd long)
+    const long long first = (long long)p.begin + base;  // global row of the first pivot
     for (int c = send + tid; c < w; c += kT) {
       double u[kS];
 #pragma unroll
       for (int q = 0; q < kS; ++q) u[q] = q < kd ? S.psave[q * W1 + c] : 0.0;
 #pragma unroll
-      for (int q = 1; q < kS; ++q) {
-        if (q < kd) {
+      for (int t = 0; t < kS - 1; ++t)
 #pragma unroll
-          for (int t = 0; t < q; ++t) u[q] = fma(-S.psave[q * W1 + base + t], u[t], u[q]);
-          S.psave[q * W1 + c] = u[q];
+        for (int q = t + 1; q < kS; ++q)
+          if (q < kd) u[q] = fma(-S.psave[q * W1 + base + t], u[t], u[q]);
+#pragma unroll
+      for (int q = 0; q < kS; ++q)
+        if (q < kd) {
+          if (q > 0) S.psave[q * W1 + c] = u[q];
+          // the solved rows to the pivot rows of this CTA
+          const long long g = first + q - row0;
+          if (g >= 0 && g < rows_here) sm[c * RP + (int)g] = u[q];
         }
-      }
     }
     __syncthreads();
-    const long long first = (long long)p.begin + base;  // global row of the first pivot
-    const int ncol = w - send;
-    // the solved rows to the pivot rows of this CTA
-    for (int e = tid; e < kd * ncol; e += kT) {
-      const int q = e / ncol, c = send + (e - q * ncol);
-      const long long g = first + q;
-      if (g >= row0 && g < row0 + rows_here) sm[c * RP + (int)(g - row0)] = S.psave[q * W1 + c];
-    }
     // f. rank-kd update of the rows below the sub-panel's pivots on the FP64
     //    tensor path (mma.sync.m16n8k4, the kd <= 8 steps as two k4 steps):
     //    warp w takes rows [32 w + 256 i, + 32) in 16 x 8 tiles over the
@@ -557,14 +578,7 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
           }
         }
     }
-    __syncthreads();  // every warp's tiles are stored
-    mine = LocalBest{0.0, -1, 0, 0.0};
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      const int r = tid + i * kT;
-      if (r < rows_here && row0 + r >= first + kd) offer_x(mine, mine_x, sm[send * RP + r], r);
-    }
-    __syncthreads();  // the next sub-panel's columns are final in shared memory
+    __syncthreads();  // every warp's tiles are stored: the next columns are final
     // released to the readers of the next sub-panel end (phase A); the
     // steps in between exchange through the transaction barriers alone
     panel::cluster_arrive();
@@ -577,7 +591,11 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
   else
     cluster.sync();
   if (timed_out) return;
-  if (rank == 0 && tid == 0) tally.flush(p.state);
+  record();
+  if (rank == 0) {
+    if (tid == 0) tally.flush(p.state);
+    for (int t = tid + (p.positioned ? 1 : 0); t < done; t += kT) p.ipiv[p.begin + t] = S.pivs[t];
+  }
 
 #pragma unroll 4
   for (int c = 0; c < w; ++c) {
@@ -615,13 +633,23 @@ size_t panel_reg_smem_bytes(int w, int rows_per_cta) {
   return reg_layout(nullptr, w, rows_per_cta, nullptr);
 }
 
-// Up to 512 rows per CTA: at 1024 (four rows per thread) the shared-memory
-// cluster panel was measured faster per column (3.9 against 4.3 us).
-int panel_reg_max_rows() { return 2 * kT; }
+// Rows per CTA and threads: a thread a row up to 512 rows, two up to 1024.  LU,
+// ms, a thread a row up to 512 / 256 threads of two rows there: n = 8192
+// 27.5 / 28.0, n = 16384 94.8 / 95.7.  Above 512 rows the shared-memory panel
+// (panel_kernel 3) was as fast (n = 16384 97.1 with it, before the changes
+// below).  What a column costs is a chain of about 3600 cycles (C = 16, 256
+// rows a CTA): stage the warps' winners 850, CTA winner and push 400, wait 520,
+// decide 460, swap and update 230, an eighth of the sub-panel's end 1100.  It
+// was 3900 while every warp reduced the CTA's winner and every thread the
+// runner-ups, the end's rows were fetched in two rounds with a division per
+// element, and each step's pivot was stored to memory.
+int panel_reg_max_rows() { return 1024; }
+int panel_reg_threads(int rows_per_cta) { return rows_per_cta <= 256 ? 256 : 512; }
 
 const void* panel_reg_kernel_for(int rows_per_cta) {
-  if (rows_per_cta <= kT) return (const void*)panel_reg_kernel<1>;
-  if (rows_per_cta <= 2 * kT) return (const void*)panel_reg_kernel<2>;
+  if (rows_per_cta <= 256) return (const void*)panel_reg_kernel<256, 1>;
+  if (rows_per_cta <= 512) return (const void*)panel_reg_kernel<512, 1>;
+  if (rows_per_cta <= 1024) return (const void*)panel_reg_kernel<512, 2>;
   return nullptr;
 }
 
