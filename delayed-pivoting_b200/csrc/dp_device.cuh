@@ -124,8 +124,9 @@ struct State {
   int block_changed;  // block rows [begin, end) whose content changed in the last panel
   Cand fallback;   // result of the last 2-D / column-fallback search
   unsigned int search_done;  // last-block-done counter of the search kernels
-  unsigned int barrier_exit; // exit counter of the panel kernel
-  int pad1[2];
+  int fallback_done;         // last-block-done counter of the fallback kernel
+  int delayed;     // 1 once a fallback search found no pivot: the factorisation ends at stop_k
+  int pad1;
   // Near-tie detector: every pivot decision (column search of a panel step,
   // fallback search) also reduces the runner-up magnitude; a decision whose
   // winner beats the runner-up by at most kNearTieC (k + 1) u |winner| (u =

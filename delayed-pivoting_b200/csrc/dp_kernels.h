@@ -180,13 +180,13 @@ void launch_search_active(const double* a, long long lda, int m, int n, int k, S
 void launch_search_nonzero_column(const double* a, long long lda, int m, int n, int k,
                                   double threshold, State* state, cudaStream_t s);
 
-// Swap full rows r1 <-> r2 over columns [0, n) and full columns c1 <-> c2 over
-// rows [0, m) (either may be a no-op when the indices are equal).
-void launch_swap_row(double* a, long long lda, int n, int r1, int r2, cudaStream_t s);
-void launch_swap_col(double* a, long long lda, int m, int c1, int c2, cudaStream_t s);
+// Ends a fallback search at step k (state->fallback): moves the pivot found to
+// (k, k) by full row and column swaps, records it and re-arms state->stop_k, or
+// sets state->delayed when no magnitude exceeds the threshold.
+void launch_apply_fallback(double* a, long long lda, int m, int n, int k, double threshold,
+                           State* state, int* ipiv, int* jpiv, cudaStream_t s);
 
 void launch_identity_records(int* ipiv, int* jpiv, int count, cudaStream_t s);
-void launch_set_record(int* ipiv, int* jpiv, int k, int p, int q, cudaStream_t s);
 
 // ---- triangular solves with many right-hand sides (trisolve.cu) ----------
 

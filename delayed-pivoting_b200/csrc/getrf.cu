@@ -582,6 +582,9 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
   Recorder& rec = *sc.r1;
   const bool la = sc.s2 != nullptr;
   const int pivots = std::min(m, n);
+  // panels enqueued without a host round trip each: with look-ahead, and where
+  // one outer block holds them all
+  const bool eq = la || pivots <= std::max(o.nb_outer, o.nb);
   rec.begin(DP_KFAM_OTHER);
   launch_identity_records(ws.d_ipiv, ws.d_jpiv, pivots, st);
   rec.end(0.0, 8.0 * pivots, 1);
@@ -594,8 +597,8 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
   const int terms = mixed_terms(o.precision);
   void* mixed_ws = terms ? ws.mixed : nullptr;
   int* const stop_word = &ws.state->stop_k;
-  std::vector<int> widths;  // the current block's panels (look-ahead)
-  if (la) DP_CHECK_CUDA(cudaMemsetAsync(stop_word, 0xFF, sizeof(int), st));  // stop_k = -1
+  std::vector<int> widths;  // the current block's panels (enqueued ones)
+  if (eq) DP_CHECK_CUDA(cudaMemsetAsync(stop_word, 0xFF, sizeof(int), st));  // stop_k = -1
   // T = I - L^{-1} of the W x W block at a(s0, s0) into buffer `which`, when
   // the block is solved by inverse (wider than the TRSM kernel's blocks);
   // returns the solve's operands for the panel stream and the other stream
@@ -629,7 +632,9 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
     if (la) DP_CHECK_CUDA(cudaMemsetAsync(ext, 0xFF, sizeof(int) * 2 * (size_t)(E - B), st));
     widths.clear();
     int b = B, e = B, stop = -1;
-    bool unread = false;  // enqueued panels whose state the host has not read
+    // enqueued panels, or a fallback's end, whose state the host has not read
+    bool unread = positioned;
+    bool over = false;  // no pivot was left at `stop`: the rest is delayed
     while (b < E) {
       int w = std::min(std::min(o.nb, ws.w_max), E - b);
       int G = 1, R = 1;
@@ -646,7 +651,7 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
       if (!use_cluster && o.panel_kernel == 1) return kInvalidArgument;
       if (!use_small && !use_cluster && !plan_panel(m - b, w, o.panel_rows, di, G, R))
         return kInvalidArgument;
-      const bool enqueue = la && (use_cluster || use_small);
+      const bool enqueue = eq && (use_cluster || use_small);
       if (!enqueue && unread) {
         // a synchronous panel follows enqueued ones: settle them first
         if (int err = read_state(hs, ws, st)) return err;
@@ -654,6 +659,7 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
         unread = false;
         if (hs.stop_k >= 0) {
           stop = hs.stop_k;
+          over = hs.delayed != 0;
           break;
         }
       }
@@ -718,7 +724,7 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
       }
       rec.end(panel_flops(m, b, w), 16.0 * (double)(m - b) * w, 1);
       positioned = false;
-      if (la) widths.push_back(w);
+      if (eq) widths.push_back(w);
 
       if (enqueue) {
         // swaps inside the block, then the rest of the block: both skip
@@ -728,9 +734,12 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
         // solved by the laswp kernel right after their permutation)
         const bool fused = w <= laswp_solve_max_width();
         rec.begin(DP_KFAM_LASWP);
-        launch_laswp(a, lda, b, w, pp.swap_block, pp.swap_extra, ws.state, B, b, e, E, st, b,
+        // (without look-ahead the swaps reach every column at once)
+        const int from = la ? B : 0, to = la ? E : n;
+        launch_laswp(a, lda, b, w, pp.swap_block, pp.swap_extra, ws.state, from, b, e, to, st, b,
                      fused ? e : 0, fused ? E : 0);
-        rec.end(fused ? (double)w * (w - 1) * (E - e) : 0.0, 16.0 * 2.0 * w * (double)(E - B - w), 1);
+        rec.end(fused ? (double)w * (w - 1) * (E - e) : 0.0,
+                16.0 * 2.0 * w * (double)(to - from - w), 1);
         update_columns(a, lda, m, b, w, e, e, E, st, rec, nullptr, nullptr, 2, stop_word, nullptr,
                        fused);
         DP_CHECK_CUDA(cudaGetLastError());
@@ -767,9 +776,16 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
     if (unread) {
       if (int err = read_state(hs, ws, st)) return err;
       if (hs.status != kOk) return hs.status;
-      if (hs.stop_k >= 0) stop = hs.stop_k;
+      if (hs.stop_k >= 0) {
+        stop = hs.stop_k;
+        over = hs.delayed != 0;
+      }
     }
-    if (stop >= 0 && la) {
+    if (over) {  // the whole active submatrix is delayed
+      info = stop;
+      break;
+    }
+    if (stop >= 0 && !widths.empty()) {
       // the panel that stopped: the last whose first column is <= stop; the
       // ones after it did nothing
       size_t p = 0;
@@ -881,21 +897,13 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
     rec.end(0.0, 8.0 * (double)(m - k) * (double)(n - k),
             o.policy == DP_POLICY_NONZERO_COLUMN ? 2 : 1);
     DP_CHECK_CUDA(cudaGetLastError());
-    if (int err = read_state(hs, ws, st)) return err;
-    if (hs.status != kOk) return hs.status;
-    const Cand c = hs.fallback;
-    if (!(c.val > o.threshold)) {
-      info = k;  // the whole active submatrix is delayed
-      break;
-    }
+    // the search's result stays on the device: the pivot moves to (k, k) and the
+    // stop word is re-armed, or everything enqueued from here on does nothing
+    // and the next read says that the rest is delayed
     rec.begin(DP_KFAM_SWAP);
-    launch_set_record(ws.d_ipiv, ws.d_jpiv, k, c.row, c.col, st);
-    launch_swap_row(a, lda, n, k, c.row, st);
-    launch_swap_col(a, lda, m, k, c.col, st);
-    rec.end(0.0, 32.0 * ((c.row != k ? (double)n : 0.0) + (c.col != k ? (double)m : 0.0)),
-            1 + (c.row != k) + (c.col != k));
+    launch_apply_fallback(a, lda, m, n, k, o.threshold, ws.state, ws.d_ipiv, ws.d_jpiv, st);
+    rec.end(0.0, 32.0 * ((double)n + (double)m), 1);
     DP_CHECK_CUDA(cudaGetLastError());
-    if (la) DP_CHECK_CUDA(cudaMemsetAsync(stop_word, 0xFF, sizeof(int), st));  // re-arm
     B = k;
     positioned = true;
   }

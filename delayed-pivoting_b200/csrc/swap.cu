@@ -9,8 +9,8 @@
 // changed, once per panel: each warp owns one column, gathers every source
 // row into registers and scatters them to their destinations.  The block
 // part of the list (destinations begin..end-1) is contiguous, so those writes
-// are coalesced.  Full-row / full-column swaps of a fallback step are
-// separate grid-stride kernels.
+// are coalesced.  The full-row and full-column swap of a fallback step are one
+// kernel that takes the pivot from the device's search result.
 #include "dp_device.cuh"
 #include "dp_kernels.h"
 
@@ -39,7 +39,8 @@ laswp_kernel(double* a, long long lda, int begin, int nblock, const int* swap_bl
   __shared__ int s_count;
   __shared__ double s_l[kSolveW * kSolveW];  // s_l[k * kSolveW + i] = L11(i, k), i > k
   const int sk = state->stop_k;
-  if (gate_begin >= 0 && sk >= 0 && sk < gate_begin) return;  // an earlier panel stopped
+  // an earlier panel stopped, or the fallback search before this one found nothing
+  if (gate_begin >= 0 && sk >= 0 && (sk < gate_begin || state->delayed)) return;
   const bool solve = s0 < s1 && sk < 0 && nblock <= kSolveW;
   const int tid = threadIdx.x;
   if (solve) {
@@ -201,23 +202,58 @@ laswp_seq_kernel(double* a, long long lda, const int* blk, const int* ext, SwapS
   }
 }
 
-__global__ void swap_row_kernel(double* a, long long lda, int n, int r1, int r2) {
-  for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n;
-       j += (long long)gridDim.x * blockDim.x) {
-    const double t = a[idx(r1, j, lda)];
-    a[idx(r1, j, lda)] = a[idx(r2, j, lda)];
-    a[idx(r2, j, lda)] = t;
+// The end of a fallback search at step k: with no magnitude above the
+// threshold the factorisation is over (state->delayed, stop_k stays); else the
+// pivot (r, c) of state->fallback moves to (k, k) - rows k <-> r over all
+// columns, then columns k <-> c over all rows, in one pass (the four elements
+// both swaps touch go to one thread) - the swap is recorded and the stop word
+// re-armed, so that the kernels enqueued behind this one run.
+__global__ void apply_fallback_kernel(double* a, long long lda, int m, int n, int k,
+                                      double threshold, State* state, int* ipiv, int* jpiv,
+                                      int* done) {
+  const Cand f = state->fallback;
+  const bool found = f.val > threshold;
+  const int r = f.row, c = f.col;
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (found) {
+    if (r != k)
+      for (int j = t0; j < n; j += step)
+        if (j != k && j != c) {
+          double *x = a + idx(k, j, lda), *y = a + idx(r, j, lda);
+          const double t = *x;
+          *x = *y;
+          *y = t;
+        }
+    if (c != k)
+      for (int i = t0; i < m; i += step)
+        if (i != k && i != r) {
+          double *x = a + idx(i, k, lda), *y = a + idx(i, c, lda);
+          const double t = *x;
+          *x = *y;
+          *y = t;
+        }
+    if (t0 == 0) {  // (r == k or c == k: the same elements under two names)
+      const double kk = a[idx(k, k, lda)], kc = a[idx(k, c, lda)];
+      const double rk = a[idx(r, k, lda)], rc = a[idx(r, c, lda)];
+      a[idx(k, k, lda)] = rc;
+      a[idx(k, c, lda)] = rk;
+      a[idx(r, k, lda)] = kc;
+      a[idx(r, c, lda)] = kk;
+      ipiv[k] = r;
+      jpiv[k] = c;
+    }
   }
-}
-
-__global__ void swap_col_kernel(double* a, long long lda, int m, int c1, int c2) {
-  double* x = a + idx(0, c1, lda);
-  double* y = a + idx(0, c2, lda);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < m;
-       i += (long long)gridDim.x * blockDim.x) {
-    const double t = x[i];
-    x[i] = y[i];
-    y[i] = t;
+  // the last CTA, once every CTA has read the search's result
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (last && threadIdx.x == 0) {
+    *done = 0;
+    if (found)
+      state->stop_k = -1;
+    else
+      state->delayed = 1;
   }
 }
 
@@ -226,11 +262,6 @@ __global__ void identity_records_kernel(int* ipiv, int* jpiv, int count) {
     ipiv[i] = i;
     jpiv[i] = i;
   }
-}
-
-__global__ void set_record_kernel(int* ipiv, int* jpiv, int k, int p, int q) {
-  ipiv[k] = p;
-  jpiv[k] = q;
 }
 
 int grid_for(long long work, int threads, int cap) {
@@ -289,21 +320,11 @@ int launch_laswp_seq(double* a, long long lda, const int* blk, const int* ext, i
   return launches;
 }
 
-void launch_swap_row(double* a, long long lda, int n, int r1, int r2, cudaStream_t s) {
-  if (r1 == r2 || n <= 0) return;
+void launch_apply_fallback(double* a, long long lda, int m, int n, int k, double threshold,
+                           State* state, int* ipiv, int* jpiv, cudaStream_t s) {
   dp::note_launch();
-  swap_row_kernel<<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(a, lda, n, r1, r2);
-}
-
-void launch_swap_col(double* a, long long lda, int m, int c1, int c2, cudaStream_t s) {
-  if (c1 == c2 || m <= 0) return;
-  dp::note_launch();
-  swap_col_kernel<<<grid_for(m, 256, 148 * 8), 256, 0, s>>>(a, lda, m, c1, c2);
-}
-
-void launch_set_record(int* ipiv, int* jpiv, int k, int p, int q, cudaStream_t s) {
-  dp::note_launch();
-  set_record_kernel<<<1, 1, 0, s>>>(ipiv, jpiv, k, p, q);
+  apply_fallback_kernel<<<grid_for(m > n ? m : n, 256, 148), 256, 0, s>>>(
+      a, lda, m, n, k, threshold, state, ipiv, jpiv, &state->fallback_done);
 }
 
 void launch_identity_records(int* ipiv, int* jpiv, int count, cudaStream_t s) {
