@@ -175,7 +175,7 @@ __device__ __forceinline__ bool beats(double v, int key, double cv, int ck) {
 // magnitude is >= 0 (a lane without a candidate offers 0 with key kNone), so
 // its bit pattern orders like its value: max of the high word, then of the
 // low word among the lanes holding that high word, then min key among the
-// lanes holding the maximum - three warp reductions.
+// lanes holding the maximum - three dependent warp reductions.
 __device__ __forceinline__ void warp_best(double v, int key, double& bv, int& bk) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(v);
   const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
@@ -183,6 +183,23 @@ __device__ __forceinline__ void warp_best(double v, int key, double& bv, int& bk
   const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
   bk = __reduce_min_sync(0xffffffffu, (hi == mhi && lo == mlo) ? key : kNone);
   bv = __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
+}
+
+// The same, and the largest of the lanes' non-negative magnitudes `w`, whose
+// reductions go between the dependent ones.
+__device__ __forceinline__ void warp_best_and_max(double v, int key, double w, double& bv, int& bk,
+                                                  double& mw) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  const unsigned long long x = (unsigned long long)__double_as_longlong(w);
+  const unsigned hi = (unsigned)(u >> 32), lo = (unsigned)u;
+  const unsigned xhi = (unsigned)(x >> 32), xlo = (unsigned)x;
+  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned whi = __reduce_max_sync(0xffffffffu, xhi);
+  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+  const unsigned wlo = __reduce_max_sync(0xffffffffu, xhi == whi ? xlo : 0u);
+  bk = __reduce_min_sync(0xffffffffu, (hi == mhi && lo == mlo) ? key : kNone);
+  bv = __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
+  mw = __longlong_as_double((long long)(((unsigned long long)whi << 32) | wlo));
 }
 
 // Largest of the lanes' non-negative magnitudes (bit-pattern order).
@@ -241,15 +258,23 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
   // the winning lane pushes its sub-panel columns j.., the reciprocal of its
   // entry in column j (computed by every lane ahead of the reductions, off
   // the path after the barrier) and the warp's result
+  // The last decision's runner-up: t_lane holds this lane's share of it until the
+  // next push, whose reductions hide it (warp 0 records, from its lane 0).
+  int t_k = -1;
+  double t_best = 0.0, t_lane = 0.0;
   auto push = [&](int j, int par, double cv, int ck, int ci, double cs) {
     double pv = 0.0;
 #pragma unroll
     for (int c = 0; c < kSb; ++c)
       if (c == j) pv = ci ? x[G::RPT - 1][c] : x[0][c];
     const double rinv = 1.0 / pv;
-    double wv;
+    double wv, second;
     int wk;
-    warp_best(cv, ck, wv, wk);
+    warp_best_and_max(cv, ck, t_lane, wv, wk, second);
+    if (warp == 0 && t_k >= 0) {
+      tally.note(t_k, t_best, second);  // (alike in every lane; one is flushed)
+      t_k = -1;
+    }
     // the warp's runner-up: the winner lane's runner-up, every other lane's best
     const double ws = warp_max_pos((wk != kNone && ck == wk) ? cs : (ck != kNone ? cv : cs));
     if (wk != kNone ? ck == wk : lane == 0) {
@@ -292,21 +317,19 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
     for (int j = 0; j < kSb; ++j) {
       if (j >= sw) break;
       const int st = base + j, par = st & 1;
+      const int q = lane & (G::kWarps - 1);  // (lanes >= kWarps repeat the others)
+      const double rv = s.rval[par][q], rs = s.rsec[par][q];
+      const int rk = s.rkey[par][q];
       double bv;
-      int bk;
-      warp_best(s.rval[par][lane & (G::kWarps - 1)], s.rkey[par][lane & (G::kWarps - 1)], bv, bk);
-      // the warp that offered the winner (keys of real candidates are unique)
-      const int bw = max(0, __ffs(__ballot_sync(0xffffffffu, lane < G::kWarps && bk != kNone &&
-                                                                s.rkey[par][lane] == bk)) - 1);
+      int key;  // logical row and warp of the winner: rows below 2^26
+      warp_best(rv, rk == kNone ? kNone : rk * kMaxWarps + q, bv, key);
+      const int bk = key == kNone ? kNone : key / kMaxWarps;
+      const int bw = key == kNone ? 0 : key % kMaxWarps;
       const bool placed = positioned && st == 0;
       if (!placed) {
-        // runner-up over the warps (lanes >= G::kWarps repeat lanes < G::kWarps)
-        const int q = lane & (G::kWarps - 1);
-        const double bs = warp_max_pos((bk != kNone && s.rkey[par][q] == bk)
-                                           ? s.rsec[par][q]
-                                           : (s.rkey[par][q] != kNone ? s.rval[par][q]
-                                                                      : s.rsec[par][q]));
-        if (tid == 0) tally.note(b + st, bk != kNone ? bv : 0.0, bs);
+        t_k = b + st;
+        t_best = bk != kNone ? bv : 0.0;
+        t_lane = bk != kNone && q == bw ? rs : (rk != kNone ? rv : rs);
       }
       if (!placed && !(bv > thr)) {
         stop = st;
@@ -351,12 +374,19 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
     const int rest = w - base - kSb;
     __syncthreads();  // psave complete
     if (kd > 0 && rest > 0) {
-      for (int c = kSb + tid; c < kSb + rest; c += G::T)
-        for (int j = 1; j < kd; ++j) {
-          double u = s.psave[j][c];
-          for (int t = 0; t < j; ++t) u = fma(-s.psave[j][t], s.psave[t][c], u);
-          s.psave[j][c] = u;
-        }
+      for (int c = kSb + tid; c < kSb + rest; c += G::T) {
+        double u[kSb];  // a step's multiples go to all later rows before the next step
+#pragma unroll
+        for (int j = 0; j < kSb; ++j) u[j] = j < kd ? s.psave[j][c] : 0.0;
+#pragma unroll
+        for (int t = 0; t < kSb - 1; ++t)
+#pragma unroll
+          for (int j = t + 1; j < kSb; ++j)
+            if (j < kd) u[j] = fma(-s.psave[j][t], u[t], u[j]);
+#pragma unroll
+        for (int j = 1; j < kSb; ++j)
+          if (j < kd) s.psave[j][c] = u[j];
+      }
       __syncthreads();
 #pragma unroll
       for (int i = 0; i < G::RPT; ++i) {
@@ -404,6 +434,10 @@ __device__ __forceinline__ int panel_regs(double* A, int n, int lda, int b, int 
       first_candidate(base, false);
       __syncthreads();
     }
+  }
+  if (warp == 0 && t_k >= 0) {  // the panel's last decision
+    const double second = warp_max_pos(t_lane);
+    tally.note(t_k, t_best, second);  // (alike in every lane; one is flushed)
   }
   // the window's remaining columns to P (physical rows)
 #pragma unroll
@@ -818,7 +852,7 @@ __device__ __forceinline__ void getrf_one(double* A, int n, int* ipiv, int* jpiv
     double bv, bs;
     int br, bc;
     active_argmax<G>(A, lda, n, k, s, bv, br, bc, bs);
-    if (tid == 0) tally.note(k, bv > 0.0 ? bv : 0.0, bv > 0.0 ? bs : 0.0);
+    tally.note(k, bv > 0.0 ? bv : 0.0, bv > 0.0 ? bs : 0.0);
     if (!(bv > thr)) {
       if (tid == 0) *info = k;
       break;

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
   auto record = [&] {
     if (rank == 0 && warp == 0 && t_k >= 0) {
       const double second = warp_max_pos(t_lane);
-      if (lane == 0) tally.note(t_k, t_best, second);
+      tally.note(t_k, t_best, second);  // (alike in every lane; one is flushed)
       t_k = -1;
     }
   };
