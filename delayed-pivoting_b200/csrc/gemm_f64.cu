@@ -273,8 +273,17 @@ using Wide8 = Cfg<64, 128, 16, 3, 2, 4, 2>;
 // 64 x 64 tiles with 32-deep k chunks in two stages, three CTAs per SM.
 using SmallK32 = Cfg<64, 64, 32, 2, 2, 2, 3>;
 
-// 0 automatic (Small4), 1 Big, 2 Half, 3 Small, 4 HalfW8, 5 Small4, 6 Wide,
-// 7 Wide8, 8 SmallK32
+// Few tiles (every update inside an outer block, its solve and the next block's
+// columns at small orders): 32 x 32 tiles, 4 warps of 16 x 16, 32-deep k chunks
+// in four stages - four times the CTAs and a third of the k loop's round trips.
+// us, Small4 -> Few: 256 x 256 x 256 17.5 -> 7.1, 1024 x 256 x 256 17.7 -> 9.8,
+// 512 x 192 x 64 7.2 -> 3.7, 100 x 68 x 32 5.1 -> 2.8; equal at 2048 x 256 x 256
+// (128 tiles of 64 x 64), slower from 256 such tiles on (1024 x 1024 x 256
+// 26.7 / 29.7).
+using Few = Cfg<32, 32, 32, 4, 2, 2, 3>;
+
+// 0 automatic (Few below one 64 x 64 tile per SM, else Small4), 1 Big, 2 Half,
+// 3 Small, 4 HalfW8, 5 Small4, 6 Wide, 7 Wide8, 8 SmallK32
 std::atomic<int> g_tile{0};
 
 }  // namespace gemm
@@ -286,7 +295,10 @@ void launch_gemm_minus(int M, int N, int K, const double* A, long long lda, cons
                        long long ldb, double* C, long long ldc, cudaStream_t s, const int* gate) {
   if (M <= 0 || N <= 0 || K <= 0) return;
   const int tile = gemm::g_tile.load(std::memory_order_relaxed);
-  if (N <= 32)
+  const long long tiles = ((M + 63LL) / 64) * ((N + 63LL) / 64);
+  if (tile == 0 && tiles < sm_count())
+    gemm::launch<gemm::Few>(M, N, K, A, lda, B, ldb, C, ldc, s, gate);
+  else if (N <= 32)
     gemm::launch<gemm::Skinny>(M, N, K, A, lda, B, ldb, C, ldc, s, gate);
   else if (tile == 1)
     gemm::launch<gemm::Big>(M, N, K, A, lda, B, ldb, C, ldc, s, gate);

@@ -177,80 +177,86 @@ void configure() {
 
 // T <- I - L^{-1} for a unit lower w x w block L (w <= 256), so that the
 // block solve X = L^{-1} B becomes the FP64 tensor-core update
-// X = B - T B (T strictly lower).  Column j of L^{-1} is one warp's forward
-// substitution L x = e_j: lane l holds rows l + 32 r, the entry x_k travels
-// by shuffle.  The CTA's 8 warps share L through shared memory: 32-column
-// chunks of its strict lower part (zeros elsewhere) are staged by cp.async,
-// the next chunk in flight while the warps step through the current one.
+// X = B - T B (T strictly lower).  Columns of L^{-1} are forward substitutions
+// L x = e_j, four to a CTA: warp r holds rows 32 r + lane of them.  Warp c
+// takes the steps of its own 32 x 32 diagonal block by shuffles, leaves its
+// entries in shared memory, and the warps below apply the 32 steps at once
+// from rows of L that they loaded while they waited.  The kernel stands
+// between two outer blocks, so its latency counts: 20.6 us at w = 256 (12.4 at
+// 128), against 36 with a warp per column and L staged through shared memory.
+// What bounds it is the chain of 256 shuffles and FMAs (some 60 cycles a step,
+// 6 us) and eight barriers with 32 steps' FMAs and loads behind each.
 constexpr int kInvMaxW = 256;
-constexpr int kInvRows = kInvMaxW / 32;  // rows per lane
-constexpr int kInvWarps = 8;
-constexpr int kInvChunk = 32;            // columns of L per staged chunk
-constexpr size_t kInvSmem = 2 * (size_t)kInvChunk * kInvMaxW * sizeof(double);
-static_assert(kInvChunk == 32, "one chunk per lane row group");
+constexpr int kInvCols = 4;  // columns per CTA
+static_assert(32 % kInvCols == 0, "a group of steps holds the diagonal");
 
-__device__ __forceinline__ void cp_async8_zfill(double* dst, const double* src, bool ok) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0)
-               : "memory");
-}
-
-__global__ void __launch_bounds__(32 * kInvWarps)
+__global__ void __launch_bounds__(kInvMaxW)
 lower_inverse_kernel(const double* __restrict__ L, long long ldl, int w, double* __restrict__ T,
                      long long ldt) {
-  extern __shared__ __align__(16) double ls[];  // [2][kInvChunk][kInvMaxW]
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int j0 = blockIdx.x * kInvWarps;
-  const int j = j0 + (tid >> 5);
-  const bool active = j < w;
-  double x[kInvRows];
+  __shared__ __align__(16) double xs[2][32][kInvCols];  // the entries of a block, by its parity
+  extern __shared__ double ds[];  // [warp][32][32]: a warp's diagonal block
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = threadIdx.x;  // the row
+  const int j = blockIdx.x * kInvCols;
+  const int c0 = j / 32, jj = j % 32;
+  const double* Li = L + i;
+  double x[kInvCols];
 #pragma unroll
-  for (int r = 0; r < kInvRows; ++r) x[r] = lane + 32 * r == j ? 1.0 : 0.0;
-  const int c_first = j0 / kInvChunk;
-  const int c_last = w >= 2 ? (w - 2) / kInvChunk : -1;  // last chunk holding a step
-  auto stage = [&](int c, int buf) {
-    double* dst = ls + (size_t)buf * kInvChunk * kInvMaxW;
-    for (int e = tid; e < kInvChunk * kInvMaxW; e += 32 * kInvWarps) {
-      const int kk = e / kInvMaxW, i = e % kInvMaxW;
-      const int k = c * kInvChunk + kk;
-      const bool ok = i < w && i > k;
-      cp_async8_zfill(dst + e, ok ? L + i + (size_t)k * (size_t)ldl : L, ok);
+  for (int u = 0; u < kInvCols; ++u) x[u] = i == j + u ? 1.0 : 0.0;
+  if (warp >= c0) {
+#pragma unroll 8
+    for (int kk = 0; kk < 32; ++kk)  // strictly lower, zeros elsewhere
+      ds[(32 * warp + kk) * 32 + lane] = lane > kk && i < w ? Li[(size_t)(32 * warp + kk) * (size_t)ldl]
+                                                             : 0.0;
+    __syncwarp();
+  }
+  for (int c = c0; 32 * c < w; ++c) {  // (CTA-uniform)
+    const int lo = c == c0 ? jj : 0;   // the block's first step
+    double l[32];
+    if (warp > c) {
+#pragma unroll
+      for (int kk = 0; kk < 32; ++kk)
+        l[kk] = i < w ? Li[(size_t)(32 * c + kk) * (size_t)ldl] : 0.0;
+    } else if (warp == c) {
+      const int hi = min(32, w - 1 - 32 * c);
+      const int first = c == c0 ? jj : -kInvCols;
+#pragma unroll 4
+      for (int kk = lo; kk < hi; ++kk) {
+        const double d = ds[(32 * c + kk) * 32 + lane];
+#pragma unroll
+        for (int u = 0; u < kInvCols; ++u) {
+          // Before column u's diagonal x_k is zero; d too, lest an infinity reach the column
+          // (selected: a branch around the shuffle makes the step seven times as long).
+          const double du = kk >= first + u ? d : 0.0;
+          x[u] = fma(-du, __shfl_sync(0xffffffffu, x[u], kk), x[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kInvCols; ++u) xs[c & 1][lane][u] = x[u];
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  if (c_first <= c_last) stage(c_first, 0);
+    __syncthreads();  // (this parity is written again after the next one)
+    if (warp > c) {
 #pragma unroll
-  for (int c = 0; c < kInvRows; ++c) {
-    if (c < c_first || c > c_last) continue;  // (CTA-uniform)
-    const int buf = (c - c_first) & 1;
-    if (c + 1 <= c_last) {
-      stage(c + 1, buf ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-    const double* lc = ls + (size_t)buf * kInvChunk * kInvMaxW;
-    if (active) {
+      for (int g = 0; g < 32; g += kInvCols) {
+        if (g < lo) continue;  // (uniform)
+        const bool past = c != c0 || g > lo;
 #pragma unroll
-      for (int kk = 0; kk < kInvChunk; ++kk) {
-        const int k = kInvChunk * c + kk;
-        if (k < j || k >= w - 1) continue;  // (warp-uniform)
-        const double xk = __shfl_sync(0xffffffffu, x[c], kk);
+        for (int t = 0; t < kInvCols; ++t) {
+          const double before = past ? l[g + t] : 0.0;  // (columns whose diagonal is still to come)
 #pragma unroll
-        for (int r = c; r < kInvRows; ++r)
-          x[r] = fma(-lc[kk * kInvMaxW + lane + 32 * r], xk, x[r]);  // zero where i <= k
+          for (int u = 0; u < kInvCols; u += 2) {
+            const double2 xk = *(const double2*)&xs[c & 1][g + t][u];
+            x[u] = fma(-(u <= t ? l[g + t] : before), xk.x, x[u]);
+            x[u + 1] = fma(-(u + 1 <= t ? l[g + t] : before), xk.y, x[u + 1]);
+          }
+        }
       }
     }
-    __syncthreads();  // this buffer is restaged two chunks later
   }
-  if (!active) return;
-  double* Tj = T + (size_t)j * (size_t)ldt;
+  if (i >= w) return;
 #pragma unroll
-  for (int r = 0; r < kInvRows; ++r) {
-    const int i = lane + 32 * r;
-    if (i < w) Tj[i] = i > j ? -x[r] : 0.0;
-  }
+  for (int u = 0; u < kInvCols; ++u)
+    if (j + u < w) T[i + (size_t)(j + u) * (size_t)ldt] = i > j + u ? -x[u] : 0.0;
 }
 
 // dst(0:rows, 0:cols) <- src(0:rows, 0:cols), both column-major: a CTA per
@@ -279,9 +285,10 @@ int lower_inverse_max_width() { return kInvMaxW; }
 void launch_lower_inverse(const double* L, long long ldl, int w, double* T, long long ldt,
                           cudaStream_t s) {
   if (w <= 0) return;
-  dp::ensure_smem((const void*)lower_inverse_kernel, kInvSmem);
+  constexpr size_t kSmem = (size_t)kInvMaxW * 32 * sizeof(double);
+  dp::ensure_smem((const void*)lower_inverse_kernel, kSmem);
   dp::note_launch();
-  lower_inverse_kernel<<<(w + kInvWarps - 1) / kInvWarps, 32 * kInvWarps, kInvSmem, s>>>(
+  lower_inverse_kernel<<<(w + kInvCols - 1) / kInvCols, (w + 31) / 32 * 32, kSmem, s>>>(
       L, ldl, w, T, ldt);
 }
 

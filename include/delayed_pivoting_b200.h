@@ -411,7 +411,7 @@ int dp_schur_update_mixed_device(int M, int N, int K, const double *A, int lda, 
                                  int ldb, double *C, int ldc, int precision, void *stream);
 
 /* Tile of that kernel for N > 32 (tuning; no result bit depends on it):
- * 0 automatic (= 5), 1 128 x 128 (one CTA per SM), 2 128 x 64 (two CTAs per
+ * 0 automatic (32 x 32 below one 64 x 64 tile per SM, at any N; else 5), 1 128 x 128 (one CTA per SM), 2 128 x 64 (two CTAs per
  * SM), 3 64 x 64 (three CTAs per SM), 4 128 x 64 with eight warps, 5 64 x 64
  * with two stages (four CTAs per SM), 6 64 x 128 with four warps, 7 64 x 128
  * with eight warps, 8 64 x 64 with 32-deep k chunks.
