@@ -60,11 +60,14 @@ struct CopyItem {  // dst = src (rows x cols)
   int rows, cols, ldd, lds;
 };
 
-size_t solve_smem(int max_n);
 int launch_orders(const int* ns, const long long* rec, const int* ipiv, const int* jpiv,
                   int* row_order, int* col_order, int count, cudaStream_t st);
-int launch_solve(const SolveItem* items, int count, int max_n, cudaStream_t st);
-int launch_residual(const ResidualItem* items, double* err, int count, int max_n, cudaStream_t st);
+int launch_solve(const SolveItem* items, int count, int max_n, int max_nrhs, cudaStream_t st);
+// Doubles per item of launch_residual's `work`: the norms and a counter, zero
+// before the first launch (each launch leaves them so).
+constexpr int kResidualWork = 3 * kMaxRhs + 8;
+int launch_residual(const ResidualItem* items, double* work, double* err, int count, int max_n,
+                    cudaStream_t st);
 int launch_axpy(const AxpyItem* items, int count, cudaStream_t st);
 int launch_copy(const CopyItem* items, int count, cudaStream_t st);
 

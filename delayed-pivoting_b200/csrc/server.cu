@@ -402,8 +402,9 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
   if (k == 0) return;
   size_t xs = 0;
   std::vector<size_t> xoff(k);
-  int max_n = 1;
+  int max_n = 1, max_nrhs = 1;
   for (int i = 0; i < k; ++i) {
+    max_nrhs = std::max(max_nrhs, items[i].nrhs);
     xoff[i] = xs;
     xs += round_up((size_t)items[i].n * items[i].nrhs, 4);
     max_n = std::max(max_n, items[i].n);
@@ -411,7 +412,7 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
   const size_t item_bytes =
       round_up(sizeof(sv::SolveItem) * k, 256) + round_up(sizeof(sv::ResidualItem) * k, 256) +
       round_up(sizeof(sv::AxpyItem) * k, 256) + round_up(sizeof(sv::CopyItem) * k, 256) +
-      round_up(sizeof(double) * k, 256);
+      round_up(sizeof(double) * k, 256) + sizeof(double) * sv::kResidualWork * (size_t)k;
   char* mem = nullptr;
   const size_t bytes = 3 * sizeof(double) * xs + item_bytes;
   auto fail = [&](int status) {
@@ -434,6 +435,11 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
   auto* d_copy = reinterpret_cast<sv::CopyItem*>(p);
   p += round_up(sizeof(sv::CopyItem) * k, 256);
   auto* d_err = reinterpret_cast<double*>(p);
+  p += round_up(sizeof(double) * k, 256);
+  auto* d_work = reinterpret_cast<double*>(p);
+  // The errors go to pinned memory where it has room: a copy to pageable memory
+  // keeps other threads out of the driver while it waits for the kernels.
+  double* const stage = static_cast<double*>(dp::pinned_stage(sizeof(double) * k));
 
   int status = DP_SUCCESS;
   auto upload = [&](void* dst, const void* src, size_t n) {
@@ -449,8 +455,10 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
     items[i].X = X + xoff[i];
     items[i].ldx = items[i].n;
   }
+  if (cudaMemsetAsync(d_work, 0, sizeof(double) * sv::kResidualWork * (size_t)k, st) != cudaSuccess)
+    status = DP_CUDA_FAILURE;
   upload(d_solve, items.data(), sizeof(sv::SolveItem) * k);
-  if (status == DP_SUCCESS) ok(sv::launch_solve(d_solve, k, max_n, st));
+  if (status == DP_SUCCESS) ok(sv::launch_solve(d_solve, k, max_n, max_nrhs, st));
 
   std::vector<int> active(k);
   for (int i = 0; i < k; ++i) active[i] = i;
@@ -464,13 +472,14 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
                                items[i].nrhs, ldas[i], jobs[i]->r.ldb, items[i].n, items[i].n};
     }
     upload(d_res, ri.data(), sizeof(sv::ResidualItem) * a);
-    if (status == DP_SUCCESS) ok(sv::launch_residual(d_res, d_err, a, max_n, st));
+    if (status == DP_SUCCESS) ok(sv::launch_residual(d_res, d_work, d_err, a, max_n, st));
     if (status == DP_SUCCESS &&
-        (cudaMemcpyAsync(err.data(), d_err, sizeof(double) * a, cudaMemcpyDeviceToHost, st) !=
-             cudaSuccess ||
+        (cudaMemcpyAsync(stage ? stage : err.data(), d_err, sizeof(double) * a,
+                         cudaMemcpyDeviceToHost, st) != cudaSuccess ||
          cudaStreamSynchronize(st) != cudaSuccess))
       status = DP_CUDA_FAILURE;
     if (status != DP_SUCCESS) break;
+    if (stage) std::copy(stage, stage + a, err.begin());
     std::vector<int> next;
     for (int q = 0; q < a; ++q) {
       const int i = active[q];
@@ -497,7 +506,7 @@ void dp_server::solve_refine(std::vector<sv::SolveItem>& items, std::vector<cons
       out[i].iterations += 1;
     }
     upload(d_solve, si.data(), sizeof(sv::SolveItem) * c);
-    if (status == DP_SUCCESS) ok(sv::launch_solve(d_solve, c, max_n, st));
+    if (status == DP_SUCCESS) ok(sv::launch_solve(d_solve, c, max_n, max_nrhs, st));
     upload(d_axpy, ai.data(), sizeof(sv::AxpyItem) * c);
     if (status == DP_SUCCESS) ok(sv::launch_axpy(d_axpy, c, st));
     active.swap(next);
@@ -600,11 +609,13 @@ void dp_server::run_small_new(std::vector<Job>& jobs, cudaStream_t st) {
                                      g->ipiv, g->jpiv, g->info, bo, st);
     if (status == DP_SUCCESS)
       status = sv::launch_orders(d_n, d_rec, g->ipiv, g->jpiv, g->row, g->col, k, st);
+    int* const stage = static_cast<int*>(dp::pinned_stage(sizeof(int) * k));
     if (status == DP_SUCCESS &&
-        (cudaMemcpyAsync(info.data(), g->info, sizeof(int) * k, cudaMemcpyDeviceToHost, st) !=
-             cudaSuccess ||
+        (cudaMemcpyAsync(stage ? stage : info.data(), g->info, sizeof(int) * k,
+                         cudaMemcpyDeviceToHost, st) != cudaSuccess ||
          cudaStreamSynchronize(st) != cudaSuccess))
       status = DP_CUDA_FAILURE;
+    if (status == DP_SUCCESS && stage) std::copy(stage, stage + k, info.begin());
   }
   std::vector<sv::SolveItem> items;
   std::vector<const Job*> sj;

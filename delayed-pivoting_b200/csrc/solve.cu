@@ -589,10 +589,13 @@ int factor_create(Factor** out, int n, const double* A, int lda, int precision, 
   if (status == kOk) {
     dp::note_launch();
     row_abs_sum_kernel<<<(n + 31) / 32, 256, 0, st>>>(A, lda, n, normA);
-    if (cudaMemcpyAsync(&f->normA, normA, sizeof(double), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
+    double* const stage = static_cast<double*>(pinned_stage(sizeof(double)));
+    if (cudaMemcpyAsync(stage ? stage : &f->normA, normA, sizeof(double), cudaMemcpyDeviceToHost,
+                        st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
       status = kCudaFailure;
+    else if (stage)
+      f->normA = *stage;
   }
   if (status == kOk) status = factorize(*f, A, lda, precision, st);
   if (status == kOk && f->precision != DP_PRECISION_FP64 && f->info == n) {
