@@ -18,8 +18,16 @@
 //            W = L D columns (:250-330) are fused, each element read and
 //            written by one thread; the materialised columns after a swap are
 //            the buffered ones re-indexed, so nothing is re-materialised.
-// Phases are separated by a grid barrier (bounded wait); every CTA makes the
-// same decision from the same buffered values.  The panel's trailing update
+// Phases are separated by a barrier; every CTA makes the same decision from the
+// same values.  Up to kClusterRows rows the CTAs are one cluster: its hardware
+// barrier, and each CTA's shared memory holds the partial maxima and the few
+// values other rows need, written there by their owners; above, a cooperative
+// grid with a counter in global memory (bounded wait) and buffers in L2.  A
+// step's time is a chain of round trips, not bandwidth: the loads of column k,
+// row p and the swap, each some 900 cycles, the barriers (600 to 900; 1800 where
+// stores drain) and the reductions.  ms, cooperative grid -> cluster with
+// integer reductions and one division per decision: n = 1000 6.7 -> 4.5,
+// 2000 14.2 -> 9.8, 3000 (two rows to a lane) 21.1 -> 16.6, 4000 29.2 -> 24.6.  The panel's trailing update
 // (finish_panel, :126-139: dsyr2k of L and W) is the lower-triangle DMMA
 // update C -= L W^T (launch_gemm_minus_lower).  W is kept transposed
 // (WT, nb x n, column i = W's row i): its row swaps move 8 * pw contiguous
@@ -34,6 +42,7 @@
 #include "dp_device.cuh"
 #include "dp_kernels.h"
 #include "dp_stats.h"
+#include "panel_argmax.cuh"
 
 namespace dp {
 namespace bk {
@@ -112,23 +121,24 @@ __device__ __forceinline__ Top2 merge(Top2 a, Top2 b) {
   return r;
 }
 
-__device__ __forceinline__ Top2 warp_top2(Top2 t) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    Top2 u;
-    u.v = __shfl_xor_sync(~0u, t.v, o);
-    u.v2 = __shfl_xor_sync(~0u, t.v2, o);
-    u.i = __shfl_xor_sync(~0u, t.i, o);
-    u.pad = 0;
-    t = merge(t, u);
-  }
-  return t;
+// The warp's largest value: magnitudes, or -1 for none (never a NaN), ordered
+// as the integers of their bits, in two integer reductions.
+__device__ __forceinline__ double warp_max(double m) {
+  const int hi = __reduce_max_sync(~0u, __double2hiint(m));
+  const unsigned lo =
+      __reduce_max_sync(~0u, __double2hiint(m) == hi ? (unsigned)__double2loint(m) : 0u);
+  return __hiloint2double(hi, (int)lo);
 }
 
-__device__ __forceinline__ double warp_max(double m) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(~0u, m, o));
-  return m;
+// merge() over the warp (lanes may repeat one another).
+__device__ __forceinline__ Top2 warp_top2(const Top2& t) {
+  Top2 r;
+  r.v = warp_max(t.v);
+  const bool holds = __double_as_longlong(t.v) == __double_as_longlong(r.v);
+  r.i = __reduce_min_sync(~0u, holds ? t.i : INT_MAX);
+  r.v2 = warp_max(holds && t.i == r.i ? t.v2 : t.v);
+  r.pad = 0;
+  return r;
 }
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
@@ -184,14 +194,12 @@ __device__ __forceinline__ void tally(double x, double y, double tol, bool& near
   if (lo > closest * hi) closest = lo / hi;
 }
 
-// stable_2x2 (delayed_sytrf_blocked.cpp:108-124); also returns |det| and the
-// threshold it is compared with.
-__device__ __forceinline__ bool stable_2x2(double a, double b, double c, double& det,
+// stable_2x2 (delayed_sytrf_blocked.cpp:108-124) of (a b; b c) / s, s the largest
+// magnitude of the three; also returns |det| and the threshold it is compared with.
+__device__ __forceinline__ bool stable_2x2(double s, double as, double bs, double cs, double& det,
                                            double& thr) {
   det = thr = 0.0;
-  const double s = fmax(fabs(a), fmax(fabs(b), fabs(c)));
   if (!(s > 0.0)) return false;
-  const double as = a / s, bs = b / s, cs = c / s;
   det = fabs(as * cs - bs * bs);
   const double nrm = fmax(fabs(as) + fabs(bs), fabs(bs) + fabs(cs));
   thr = kDetTol * nrm * nrm;
@@ -272,8 +280,31 @@ __device__ __forceinline__ void set_entry(double (&lr)[kQ], int q, int j, double
     if (t == tj) lr[t] = v;
 }
 
-template <int RPT>
+// What a cluster's CTAs leave in each other's shared memory: a partial per CTA
+// and the values of a step that the rows' owners hold.
+constexpr int kMaxCluster = 16;
+struct Shared {
+  Top2 cpart[kMaxCluster];
+  double rpart[kMaxCluster];
+  double dkk, dpp, d10, rowk, rowk1, colk1;
+};
+
+__device__ __forceinline__ void st_peer(const double* local, int rank, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(
+                   panel::peer_addr(panel::smem_addr(local), rank)),
+               "d"(v)
+               : "memory");
+}
+__device__ __forceinline__ void st_peer(const int* local, int rank, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(
+                   panel::peer_addr(panel::smem_addr(local), rank)),
+               "r"(v)
+               : "memory");
+}
+
+template <int RPT, bool kCluster>
 __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int parity) {
+  __shared__ Shared sh;
   __shared__ double s_w[kMaxNb];
   __shared__ Top2 s_t[kWarps];
   __shared__ double s_m[kWarps];
@@ -299,6 +330,7 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
   const long long gstride = (long long)G * kThreads;
   unsigned long long checked = 0, nnear = 0;
   double closest = 0.0;
+  const bool keeps_tally = blockIdx.x == 0 && warp == kWarps - 1;
 
   long long rowi[RPT];
   double lr[RPT][kQ], cv[RPT], rv[RPT], av[RPT], a1[RPT];
@@ -310,6 +342,22 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
     for (int t = 0; t < kQ; ++t) lr[s][t] = 0.0;
   }
   long long rl0 = -1, rl1 = -1;  // rows whose cached entries are reloaded before phase A
+  const int me = blockIdx.x;     // (a cluster is the whole grid)
+  auto barrier = [&]() -> bool {
+    if constexpr (kCluster) {
+      panel::cluster_arrive();
+      panel::cluster_wait();
+      return true;
+    } else {
+      return grid_barrier(ctr, target, &st->status, &s_ok);
+    }
+  };
+  // A value for all CTAs.  One of a step is read after the next barrier, and
+  // written again in the next step, after a further one.
+  auto tell = [&](const double* where, double v) {
+    for (int r = 0; r < G; ++r) st_peer(where, r, v);
+  };
+  if (kCluster) barrier();  // every CTA runs before the first store into its memory
 
   while (k < e && pw < P.nb) {
     // ---- phase A: column k of the panel-updated matrix, top-2 below the diagonal
@@ -328,7 +376,8 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
       cv[s] = v;
       const long long i = rowi[s];
       if (q == 0 && i >= k && i < n) {
-        P.col[i] = v;
+        if (!kCluster) P.col[i] = v;
+        if (kCluster && i == k) tell(&sh.dkk, v);
         if (i > k && i < e) consider(t, fabs(v), (int)i);
       }
     }
@@ -336,15 +385,26 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
     if (lane == 0) s_t[warp] = t;
     __syncthreads();
     if (warp == 0) {
-      Top2 u = lane < kWarps ? s_t[lane] : Top2{-1.0, -1.0, INT_MAX, 0};
+      Top2 u = s_t[lane % kWarps];
       u = warp_top2(u);
-      if (lane == 0) P.cpart[blockIdx.x] = u;
+      if (kCluster) {
+        if (lane < G) {
+          st_peer(&sh.cpart[me].v, lane, u.v);
+          st_peer(&sh.cpart[me].v2, lane, u.v2);
+          st_peer(&sh.cpart[me].i, lane, u.i);
+        }
+      } else if (lane == 0) {
+        P.cpart[blockIdx.x] = u;
+      }
     }
-    if (!grid_barrier(ctr, target, &st->status, &s_ok)) return;
+    if (!barrier()) return;
 
     // ---- phase B: the decision's inputs (every CTA reduces the same partials)
-    const double dkk = ld(P.col + k);  // issued before the partials' loads: one round trip
-    if (warp == 0) {
+    const double dkk = kCluster ? sh.dkk : ld(P.col + k);  // before the partials' loads: one round trip
+    Top2 best;
+    if (kCluster) {
+      best = warp_top2(sh.cpart[lane % G]);
+    } else if (warp == 0) {
       // all of the lane's partials in flight at once (G <= 32 kPartsPerLane)
       Top2 c[kPartsPerLane];
 #pragma unroll
@@ -363,8 +423,10 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
       u = warp_top2(u);
       if (lane == 0) s_best = u;
     }
-    __syncthreads();
-    const Top2 best = s_best;
+    if (!kCluster) {
+      __syncthreads();
+      best = s_best;
+    }
     int p = k;
     double colmax = 0.0;
     if (e - k > 1) {
@@ -399,7 +461,18 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
         rv[s] = v;
         const long long i = rowi[s];
         if (q == 0 && i >= k && i < n) {
-          P.row[i] = v;
+          if (!kCluster) P.row[i] = v;
+          if (kCluster) {  // what the decision and phase C read from other rows
+            if (i == p) {
+              tell(&sh.dpp, v);
+              tell(&sh.d10, cv[s]);
+            }
+            if (i == k) tell(&sh.rowk, v);
+            if (i == k + 1) {
+              tell(&sh.rowk1, v);
+              tell(&sh.colk1, cv[s]);
+            }
+          }
           if (i < e && i != p) m = fmax(m, fabs(v));
         }
       }
@@ -407,21 +480,27 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
       if (lane == 0) s_m[warp] = m;
       __syncthreads();
       if (warp == 0) {
-        double u = lane < kWarps ? s_m[lane] : 0.0;
+        double u = s_m[lane % kWarps];
         u = warp_max(u);
-        if (lane == 0) P.rpart[blockIdx.x] = u;
+        if (kCluster) {
+          if (lane < G) st_peer(&sh.rpart[me], lane, u);
+        } else if (lane == 0) {
+          P.rpart[blockIdx.x] = u;
+        }
       }
-      if (!grid_barrier(ctr, target, &st->status, &s_ok)) return;
+      if (!barrier()) return;
       // every value the decision and phase C read from other rows, issued
       // with the partials' loads: one round trip
-      dpp = ld(P.row + p);
-      d10 = ld(P.col + p);
-      rowk = ld(P.row + k);
+      dpp = kCluster ? sh.dpp : ld(P.row + p);
+      d10 = kCluster ? sh.d10 : ld(P.col + p);
+      rowk = kCluster ? sh.rowk : ld(P.row + k);
       if (k + 1 < n) {
-        rowk1 = ld(P.row + k + 1);
-        colk1 = ld(P.col + k + 1);
+        rowk1 = kCluster ? sh.rowk1 : ld(P.row + k + 1);
+        colk1 = kCluster ? sh.colk1 : ld(P.col + k + 1);
       }
-      if (warp == 0) {
+      if (kCluster) {
+        rowmax = warp_max(sh.rpart[lane % G]);
+      } else if (warp == 0) {
         double c[kPartsPerLane];
 #pragma unroll
         for (int r = 0; r < kPartsPerLane; ++r)
@@ -432,41 +511,61 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
         u = warp_max(u);
         if (lane == 0) s_rowmax = u;
       }
-      __syncthreads();
-      rowmax = s_rowmax;
+      if (!kCluster) {
+        __syncthreads();
+        rowmax = s_rowmax;
+      }
     }
 
-    // ---- the decision (delayed_sytrf_blocked.cpp:192-235), identical in every CTA
+    // ---- the decision (delayed_sytrf_blocked.cpp:192-235), identical in every
+    // warp.  Its four quotients are one division, a lane each: (dkk, d10, dpp)
+    // over the largest of them, and colmax / rowmax.
     const double app = fabs(dpp);
-    const double tol = 4.0 * (double)(k + 1) * kUnit;
-    bool near = false;
-    if (best.v2 >= 0.0) tally(best.v2, best.v, tol, near, closest);
     int kind = kDelay;
-    double det = 0.0, thr = 0.0;
+    double det = 0.0, thr = 0.0, c2r = 0.0, scale = 0.0, s00 = 0.0, s10 = 0.0, s11 = 0.0;
+    bool c2 = false, c3 = false;
     if (any) {
-      tally(akk, kAlpha * colmax, tol, near, closest);
       if (c1) {
         kind = kOne;
       } else {
-        const double c2r = kAlpha * colmax * (colmax / rowmax);
-        tally(akk, c2r, tol, near, closest);
-        if (akk >= c2r) {
+        scale = fmax(fabs(dkk), fmax(fabs(d10), app));
+        const double x = lane == 0 ? dkk : lane == 1 ? d10 : lane == 2 ? dpp : colmax;
+        const double ratio = x / (lane < 3 ? scale : rowmax);
+        s00 = __shfl_sync(~0u, ratio, 0);
+        s10 = __shfl_sync(~0u, ratio, 1);
+        s11 = __shfl_sync(~0u, ratio, 2);
+        c2r = kAlpha * colmax * __shfl_sync(~0u, ratio, 3);
+        c2 = akk >= c2r;
+        c3 = !c2 && app >= kAlpha * rowmax;
+        if (c2) {
           kind = kOne;
-        } else {
-          tally(app, kAlpha * rowmax, tol, near, closest);
-          if (app >= kAlpha * rowmax) {
-            kind = kOneSwap;
-          } else {
-            const bool ok2 = stable_2x2(dkk, d10, dpp, det, thr);
-            tally(det, thr, tol, near, closest);
-            if (ok2) kind = pw + 2 > P.nb ? kBreak : kTwo;
-          }
+        } else if (c3) {
+          kind = kOneSwap;
+        } else if (stable_2x2(scale, s00, s10, s11, det, thr)) {
+          kind = pw + 2 > P.nb ? kBreak : kTwo;
         }
       }
     }
-    if (kind != kBreak) {  // counted by thread 0 of CTA 0; every thread tracks `closest`
-      ++checked;
-      if (near) ++nnear;
+    // the near-tie record, by one warp of one CTA (a step that breaks is counted
+    // by the next panel, which takes it again)
+    if (keeps_tally) {
+      const double tol = 4.0 * (double)(k + 1) * kUnit;
+      bool near = false;
+      if (best.v2 >= 0.0) tally(best.v2, best.v, tol, near, closest);
+      if (any) {
+        tally(akk, kAlpha * colmax, tol, near, closest);
+        if (!c1) {
+          tally(akk, c2r, tol, near, closest);
+          if (!c2) {
+            tally(app, kAlpha * rowmax, tol, near, closest);
+            if (!c3) tally(det, thr, tol, near, closest);
+          }
+        }
+      }
+      if (kind != kBreak) {
+        ++checked;
+        if (near) ++nnear;
+      }
     }
     if (kind == kBreak) break;  // the 2x2 block starts the next panel (:245-248)
 
@@ -554,9 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
     } else {  // kTwo: x = k + 1, y = p; columns k, k + 1 from `col`, `row`
       const bool sw = p != k + 1;
       const double d00 = dkk, d11 = dpp;
-      const double sc = fmax(fabs(d00), fmax(fabs(d10), fabs(d11)));
-      const double s00 = d00 / sc, s10 = d10 / sc, s11 = d11 / sc;
-      const double inv = 1.0 / (sc * (s00 * s11 - s10 * s10));
+      const double inv = 1.0 / (scale * (s00 * s11 - s10 * s10));
       const long long k1 = k + 1;
       if (gt == gstride - 1) {
         P.piv[k] = 2;
@@ -612,10 +709,10 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
       pw += 2;
     }
     if (k < e && pw < P.nb) {
-      if (!grid_barrier(ctr, target, &st->status, &s_ok)) return;
+      if (!barrier()) return;
     }
   }
-  if (blockIdx.x == 0 && tid == 0) {
+  if (keeps_tally && lane == 0) {
     st->k = k;
     st->e = e;
     st->checked += checked;
@@ -628,14 +725,19 @@ __global__ void __launch_bounds__(kThreads, 1) bk_panel_kernel(Params P, int par
 constexpr int kMaxSlots = 4;
 const void* panel_kernel_for(int slots) {
   switch (slots) {
-    case 1: return (const void*)bk_panel_kernel<1>;
-    case 2: return (const void*)bk_panel_kernel<2>;
+    case 1: return (const void*)bk_panel_kernel<1, false>;
+    case 2: return (const void*)bk_panel_kernel<2, false>;
     case 3:
-    case 4: return (const void*)bk_panel_kernel<4>;
+    case 4: return (const void*)bk_panel_kernel<4, false>;
     default: return nullptr;
   }
 }
 
+constexpr int kClusterSlots = 2;
+constexpr int kClusterRows = kMaxCluster * kRowsPerCta * kClusterSlots;
+const void* cluster_kernel_for(int slots) {
+  return slots <= 1 ? (const void*)bk_panel_kernel<1, true> : (const void*)bk_panel_kernel<2, true>;
+}
 
 __global__ void bk_init_kernel(int n, int* perm, int* piv, State* st) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -666,10 +768,50 @@ int panel_ctas_max() {
   int sms = 0, coop = 0, per = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-  if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bk::bk_panel_kernel<4>,
+  if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, bk::bk_panel_kernel<4, false>,
                                                               bk::kThreads, 0) != cudaSuccess)
     return 0;
   return per > 0 ? sms : 0;
+}
+
+cudaError_t launch_cluster_panel(int slots, int ctas, void** args, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(bk::kThreads);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, bk::cluster_kernel_for(slots), args);
+}
+
+// Whether the device holds the largest cluster of the panel kernel.
+bool cluster_panel_available() {
+  for (int slots = 1; slots <= bk::kClusterSlots; ++slots)
+    if (cudaFuncSetAttribute(bk::cluster_kernel_for(slots),
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = bk::kMaxCluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(bk::kMaxCluster);
+  cfg.blockDim = dim3(bk::kThreads);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, bk::cluster_kernel_for(bk::kClusterSlots), &cfg) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return clusters > 0;
 }
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -742,6 +884,8 @@ int sytrf_device(int n, double* d_a, int lda, int* perm, int* piv_size, int* inf
   rec.end(0.0, 8.0 * n + sizeof(bk::State), 1);
   if (cudaGetLastError() != cudaSuccess) status = kCudaFailure;
   int pb = 0, e = n, parity = 0;
+  // a caller's grid is a cooperative one
+  const bool clusters = grid == 0 && cluster_panel_available();
   while (status == kOk) {
     void* args[] = {(void*)&P, (void*)&parity};
     note_launch();
@@ -749,8 +893,17 @@ int sytrf_device(int n, double* d_a, int lda, int* perm, int* piv_size, int* inf
     const long long per_slot = (long long)G * bk::kRowsPerCta;
     const int slots = (int)((n - pb + per_slot - 1) / per_slot);
     void* const stage = pinned_stage(sizeof(bk::State));
-    if (cudaLaunchCooperativeKernel(bk::panel_kernel_for(slots), dim3(G), dim3(bk::kThreads), args,
-                                    0, s) != cudaSuccess ||
+    // A cluster while it holds the rows, of as many CTAs (a power of two) as rows
+    // of one slot, at most 16.
+    int ctas = 1;
+    while (ctas < bk::kMaxCluster && ctas * bk::kRowsPerCta < n - pb) ctas *= 2;
+    const cudaError_t launched =
+        clusters && n - pb <= bk::kClusterRows
+            ? launch_cluster_panel((n - pb + ctas * bk::kRowsPerCta - 1) /
+                                       (ctas * bk::kRowsPerCta), ctas, args, s)
+            : cudaLaunchCooperativeKernel(bk::panel_kernel_for(slots), dim3(G),
+                                          dim3(bk::kThreads), args, 0, s);
+    if (launched != cudaSuccess ||
         cudaMemcpyAsync(stage ? stage : h, P.st, sizeof(bk::State), cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
