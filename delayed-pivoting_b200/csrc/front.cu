@@ -118,21 +118,34 @@ std::vector<int> composite(const int* rec, int count, int size) {
 }  // namespace
 }  // namespace front
 
+// Columns (rows of U12) that a solve finishes before it updates all that follow:
+// updates of depth 32 or 64 over the whole remainder are bound by the traffic of
+// C (2048 x 1024 x 32: 20 us for 5 us of arithmetic).
+constexpr int kSolveOuter = 256;
+
 // Right-side solve X = B U^{-1} for B rows x w (column-major, ldb) and U the
 // w x w upper triangle at u (ldu): 32-column blocks, each solved per row and
-// then subtracted from the columns after it by the DMMA update.
+// then subtracted from the columns after it by the DMMA update, within outer
+// blocks of 256 columns.
 void rsolve_upper(double* B, long long ldb, int rows, int w, const double* U, long long ldu,
                   cudaStream_t st) {
   if (rows <= 0 || w <= 0) return;
-  for (int j0 = 0; j0 < w; j0 += front::kSolveW) {
-    const int wb = std::min(front::kSolveW, w - j0);
-    dp::note_launch();
-    front::rsolve_upper_kernel<<<(rows + front::kThreads - 1) / front::kThreads, front::kThreads,
-                                 0, st>>>(B + idx(0, j0, ldb), ldb, rows, wb,
-                                          U + idx(j0, j0, ldu), ldu);
-    if (j0 + wb < w)
-      launch_gemm_minus(rows, w - j0 - wb, wb, B + idx(0, j0, ldb), ldb,
-                        U + idx(j0, j0 + wb, ldu), ldu, B + idx(0, j0 + wb, ldb), ldb, st);
+  auto update = [&](int j, int wj, int c0, int c1) {  // columns [c0, c1) by [j, j + wj)
+    if (c0 < c1)
+      launch_gemm_minus(rows, c1 - c0, wj, B + idx(0, j, ldb), ldb, U + idx(j, c0, ldu), ldu,
+                        B + idx(0, c0, ldb), ldb, st);
+  };
+  for (int o0 = 0; o0 < w; o0 += kSolveOuter) {
+    const int o1 = std::min(w, o0 + kSolveOuter);
+    for (int j0 = o0; j0 < o1; j0 += front::kSolveW) {
+      const int wb = std::min(front::kSolveW, o1 - j0);
+      dp::note_launch();
+      front::rsolve_upper_kernel<<<(rows + front::kThreads - 1) / front::kThreads,
+                                   front::kThreads, 0, st>>>(B + idx(0, j0, ldb), ldb, rows, wb,
+                                                             U + idx(j0, j0, ldu), ldu);
+      update(j0, wb, j0 + wb, o1);
+    }
+    update(o0, o1 - o0, o1, w);
   }
 }
 
@@ -142,6 +155,8 @@ namespace dp {
 
 int getrf_device(int m, int n, double* d_a, int lda, int* ipiv, int* jpiv, int* info,
                  cudaStream_t st, const dp_options* opt);
+cudaStream_t fork_lane(cudaStream_t st);
+int join_lane(cudaStream_t lane, cudaStream_t st);
 
 namespace front {
 
@@ -173,15 +188,26 @@ int finish(int m, int n, int p, int k, double* F, long long ldf, const int* ip, 
     launch_copy_block(tmp, mr, F + idx(p, 0, ldf), ldf, mr, p, st);
   }
   if (k > 0) {
-    // 3. U12 = L11^{-1} F12 in 64-row blocks, then the delayed rows of F12
+    // 3. U12 = L11^{-1} F12 in 64-row blocks within outer blocks of 256, then the
+    // delayed rows of F12.  It shares nothing with step 4, whose kernels leave as
+    // much of the device idle: the two run side by side.
+    const bool both = nr > 0 && mr > 0;
+    cudaStream_t s3 = both ? fork_lane(st) : st;
     if (nr > 0) {
       const int tw = trsm_max_width();
-      for (int b = 0; b < k; b += tw) {
-        const int wb = std::min(tw, k - b);
-        launch_trsm_unit_lower(F, ldf, b, wb, p, nr, st);
-        if (b + wb < p)  // rows after the block: the rest of U12 and the delayed rows
-          launch_gemm_minus(p - b - wb, nr, wb, F + idx(b + wb, b, ldf), ldf, F + idx(b, p, ldf),
-                            ldf, F + idx(b + wb, p, ldf), ldf, st);
+      auto update = [&](int b, int wb, int r0, int r1) {  // rows [r0, r1) by [b, b + wb)
+        if (r0 < r1)
+          launch_gemm_minus(r1 - r0, nr, wb, F + idx(r0, b, ldf), ldf, F + idx(b, p, ldf), ldf,
+                            F + idx(r0, p, ldf), ldf, s3);
+      };
+      for (int o0 = 0; o0 < k; o0 += kSolveOuter) {
+        const int o1 = std::min(k, o0 + kSolveOuter);
+        for (int b = o0; b < o1; b += tw) {
+          const int wb = std::min(tw, o1 - b);
+          launch_trsm_unit_lower(F, ldf, b, wb, p, nr, s3);
+          update(b, wb, b + wb, o1);
+        }
+        update(o0, o1 - o0, o1, p);  // the rest of U12 and the delayed rows
       }
     }
     if (mr > 0) {
@@ -190,6 +216,10 @@ int finish(int m, int n, int p, int k, double* F, long long ldf, const int* ip, 
       if (p > k)
         launch_gemm_minus(mr, p - k, k, F + idx(p, 0, ldf), ldf, F + idx(0, k, ldf), ldf,
                           F + idx(p, k, ldf), ldf, st);
+    }
+    const int joined = s3 != st ? join_lane(s3, st) : kOk;
+    if (joined != kOk) return joined;
+    if (mr > 0) {
       // 5. the rest of the front
       if (nr > 0)
         launch_gemm_minus(mr, nr, k, F + idx(p, 0, ldf), ldf, F + idx(0, p, ldf), ldf,

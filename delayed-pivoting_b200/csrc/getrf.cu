@@ -511,6 +511,31 @@ Lanes* lanes_for_device() {
   return &l;
 }
 
+}  // namespace
+
+// A stream of this thread's that continues `st` here; `st` itself when there is none.
+cudaStream_t fork_lane(cudaStream_t st) {
+  Lanes* const l = lanes_for_device();
+  if (!l || cudaEventRecord(l->fork, st) != cudaSuccess ||
+      cudaStreamWaitEvent(l->left, l->fork, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return st;
+  }
+  return l->left;
+}
+
+// `st` continues after `lane` (a fork_lane() of this thread).
+int join_lane(cudaStream_t lane, cudaStream_t st) {
+  Lanes* const l = lanes_for_device();
+  if (l && cudaEventRecord(l->join, lane) == cudaSuccess &&
+      cudaStreamWaitEvent(st, l->join, 0) == cudaSuccess)
+    return kOk;
+  cudaGetLastError();
+  return cudaStreamSynchronize(lane) == cudaSuccess ? kOk : kCudaFailure;
+}
+
+namespace {
+
 // Where factorize issues its work: `s1` always; `s2` (look-ahead) takes the
 // trailing updates right of the next outer block, ordered against `s1` by
 // the events `block` (s1 -> s2: an outer block and the next block's columns
