@@ -418,8 +418,8 @@ int dp_schur_update_mixed_device(int M, int N, int K, const double *A, int lda, 
  * Returns the previous setting, or -1 for an invalid one. */
 int dp_gemm_tile(int tile);
 
-/* CTAs of one triangular-solve launch of the solve / refinement path (tuning;
- * no result bit depends on it): 0 automatic (min(row blocks, SMs)), g > 0 at
+/* CTAs of a solve's launch (both sweeps; solves and refinement; tuning, no
+ * result bit depends on it): 0 automatic (min(row blocks, SMs)), g > 0 at
  * most g, g < 0 one CTA per -g blocks of 64 rows (at most 32).  Returns the
  * previous setting, or -2000 for a setting outside [-1024, 1024]. */
 int dp_tri_solve_grid(int policy);
