@@ -929,6 +929,7 @@ __global__ void __launch_bounds__(G::T, G::MINB) batched_getrf_kernel(Params p) 
 // the swap lists the laswp kernel applies outside the panel.
 template <class G>
 __global__ void __launch_bounds__(G::T, 1) panel_small_kernel(PanelParams p) {
+  after_previous_kernel();
   // every thread reads the same word before any barrier or state write
   if (p.gated && p.state->stop_k >= 0) return;
   extern __shared__ __align__(16) double dsm[];
@@ -1151,7 +1152,7 @@ int launch_panel_small(const PanelParams& pp, cudaStream_t st) {
     using G = decltype(geo);
     if (!ensure_smem((const void*)batch::panel_small_kernel<G>, smem)) return kCudaFailure;
     note_launch();
-    batch::panel_small_kernel<G><<<1, G::T, smem, st>>>(pp);
+    launch_behind(batch::panel_small_kernel<G>, dim3(1), G::T, smem, st, pp);
     return kOk;
   };
   const int rc = rows <= 128   ? go(batch::PanelGeo<128>{})

@@ -229,4 +229,10 @@ __device__ __forceinline__ int ld_volatile_i32(const int* p) {
   return v;
 }
 
+// First statement of a kernel that launch_behind() starts: waits for the kernel
+// before it on the stream and its writes (nothing to wait for in a plain launch).
+__device__ __forceinline__ void after_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 }  // namespace dp

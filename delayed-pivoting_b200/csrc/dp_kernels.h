@@ -238,4 +238,27 @@ void factor_destroy(Factor* f, cudaStream_t st);
 int factor_condest(Factor* f, const double* A, int lda, double* kappa, double* inv_norm,
                    cudaStream_t st);
 
+// Launches a kernel that begins with after_previous_kernel(): its CTAs are in
+// place when the last of the kernel before it on the stream has left, instead of
+// being sent then.  The panels' chains of short kernels lose about 1 us at each
+// link: LU n = 1024 2.09 -> 1.92 ms, 2048 4.61 -> 4.35, 8192 26.5 -> 25.7.  Plain
+// under capture.
+template <class... P, class... Q>
+void launch_behind(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                   Q... args) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(st, &capture);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace dp

@@ -63,6 +63,7 @@ __global__ void gather_cols_kernel(const double* __restrict__ a, long long lda, 
 __global__ void __launch_bounds__(kThreads)
 rsolve_upper_kernel(double* __restrict__ B, long long ldb, int rows, int w,
                     const double* __restrict__ U, long long ldu) {
+  after_previous_kernel();
   __shared__ double us[kSolveW * kSolveW];  // us[j * kSolveW + i] = U(i, j), i <= j
   __shared__ double rinv[kSolveW];
   for (int e = threadIdx.x; e < kSolveW * kSolveW; e += blockDim.x) {
@@ -140,9 +141,9 @@ void rsolve_upper(double* B, long long ldb, int rows, int w, const double* U, lo
     for (int j0 = o0; j0 < o1; j0 += front::kSolveW) {
       const int wb = std::min(front::kSolveW, o1 - j0);
       dp::note_launch();
-      front::rsolve_upper_kernel<<<(rows + front::kThreads - 1) / front::kThreads,
-                                   front::kThreads, 0, st>>>(B + idx(0, j0, ldb), ldb, rows, wb,
-                                                             U + idx(j0, j0, ldu), ldu);
+      launch_behind(front::rsolve_upper_kernel,
+                    dim3((rows + front::kThreads - 1) / front::kThreads), front::kThreads, 0, st,
+                    B + idx(0, j0, ldb), ldb, rows, wb, U + idx(j0, j0, ldu), ldu);
       update(j0, wb, j0 + wb, o1);
     }
     update(o0, o1 - o0, o1, w);

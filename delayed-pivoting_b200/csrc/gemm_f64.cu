@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 dgemm_minus_kernel(int M, int N, int K, const double* __restrict__ A, long long lda,
                    const double* __restrict__ B, long long ldb, double* Cm, long long ldc,
                    const int* gate, bool lower) {
+  dp::after_previous_kernel();
   if (gate && *gate >= 0) return;  // an enqueued panel sequence stopped before this update
   long long m0, n0;
   if (lower) {
@@ -241,8 +242,8 @@ void launch(int M, int N, int K, const double* A, long long lda, const double* B
     }
   }
   dp::note_launch();
-  dgemm_minus_kernel<C>
-      <<<grid, C::THREADS, C::SMEM, s>>>(M, N, K, A, lda, B, ldb, Cm, ldc, gate, lower);
+  dp::launch_behind(dgemm_minus_kernel<C>, grid, C::THREADS, C::SMEM, s, M, N, K, A, lda, B, ldb,
+                    Cm, ldc, gate, lower);
 }
 
 // 128 x 128 tiles, 8 warps of 64 x 32, one CTA per SM (212 KB of stages).

@@ -720,7 +720,9 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
         if (int err = launch_panel_small(pp, st)) return err;
       } else if (use_cluster) {
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];  // (the register panel: launch_behind())
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = G;
         attr[0].val.clusterDim.y = 1;
@@ -731,7 +733,7 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
             use_reg ? panel_reg_smem_bytes(w, R) : panel_cluster_smem_bytes(w, R);
         cfg.stream = st;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = use_reg ? 2 : 1;
         dp::note_launch();
         if (use_reg) {
           void* args[] = {&pp};

@@ -136,6 +136,7 @@ __host__ __device__ inline size_t reg_layout(unsigned char* base, int w, int R, 
 template <int kT, int RPT>
 __global__ void __launch_bounds__(kT, 1) panel_reg_kernel(PanelParams p) {
   constexpr int kW = kT / 32;
+  after_previous_kernel();
   // Every CTA reads the same word before any barrier or state write (a stop
   // is recorded only by an earlier kernel), so all of them leave together.
   if (p.gated && p.state->stop_k >= 0) return;

@@ -38,6 +38,7 @@ laswp_kernel(double* a, long long lda, int begin, int nblock, const int* swap_bl
   __shared__ int s_src[kMaxSwapEntries];
   __shared__ int s_count;
   __shared__ double s_l[kSolveW * kSolveW];  // s_l[k * kSolveW + i] = L11(i, k), i > k
+  after_previous_kernel();
   const int sk = state->stop_k;
   // an earlier panel stopped, or the fallback search before this one found nothing
   if (gate_begin >= 0 && sk >= 0 && (sk < gate_begin || state->delayed)) return;
@@ -281,8 +282,8 @@ void launch_laswp(double* a, long long lda, int begin, int nblock, const int* sw
   const int warps = kLaswpThreads / 32;
   const int grid = grid_for(ncols, warps, 148 * 16);
   dp::note_launch();
-  laswp_kernel<<<grid, kLaswpThreads, 0, s>>>(a, lda, begin, nblock, swap_block, swap_extra,
-                                              state, c0, c1, c2, c3, gate_begin, s0, s1);
+  launch_behind(laswp_kernel, dim3(grid), kLaswpThreads, 0, s, a, lda, begin, nblock, swap_block,
+                swap_extra, state, c0, c1, c2, c3, gate_begin, s0, s1);
 }
 
 int laswp_solve_max_width() { return kSolveW; }

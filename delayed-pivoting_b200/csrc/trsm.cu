@@ -47,6 +47,7 @@ __device__ __forceinline__ void stage_out(double* B, long long ldb, int w, int n
 __global__ void __launch_bounds__(kTrsmThreads)
 trsm_lower_unit_kernel(const double* __restrict__ L, long long ldl, double* B, long long ldb, int w,
                        int nc, const int* gate) {
+  after_previous_kernel();
   if (gate && *gate >= 0) return;
   extern __shared__ __align__(16) double tsm[];
   double* Ls = tsm;                    // Ls[p * 64 + i] = L(i, p), zero outside the strict lower part
@@ -196,6 +197,7 @@ lower_inverse_kernel(const double* __restrict__ L, long long ldl, int w, double*
   __shared__ __align__(16) double xs[2][32][kInvCols];  // the entries of a block, by its parity
   extern __shared__ double ds[];  // [warp][32][32]: a warp's diagonal block
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  after_previous_kernel();
   const int i = threadIdx.x;  // the row
   const int j = blockIdx.x * kInvCols;
   const int c0 = j / 32, jj = j % 32;
@@ -264,6 +266,7 @@ lower_inverse_kernel(const double* __restrict__ L, long long ldl, int w, double*
 __global__ void __launch_bounds__(256)
 copy_block_kernel(const double* __restrict__ src, long long lds, double* __restrict__ dst,
                   long long ldd, int rows, int cols) {
+  after_previous_kernel();
   for (long long c = blockIdx.x; c < cols; c += gridDim.x) {
     const double* s = src + c * lds;
     double* d = dst + c * ldd;
@@ -277,7 +280,8 @@ void launch_copy_block(const double* src, long long lds, double* dst, long long 
                        int cols, cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return;
   dp::note_launch();
-  copy_block_kernel<<<std::min(cols, 148 * 8), 256, 0, s>>>(src, lds, dst, ldd, rows, cols);
+  launch_behind(copy_block_kernel, dim3(std::min(cols, 148 * 8)), 256, 0, s, src, lds, dst, ldd, rows,
+                cols);
 }
 
 int lower_inverse_max_width() { return kInvMaxW; }
@@ -288,8 +292,8 @@ void launch_lower_inverse(const double* L, long long ldl, int w, double* T, long
   constexpr size_t kSmem = (size_t)kInvMaxW * 32 * sizeof(double);
   dp::ensure_smem((const void*)lower_inverse_kernel, kSmem);
   dp::note_launch();
-  lower_inverse_kernel<<<(w + kInvCols - 1) / kInvCols, (w + 31) / 32 * 32, kSmem, s>>>(
-      L, ldl, w, T, ldt);
+  launch_behind(lower_inverse_kernel, dim3((w + kInvCols - 1) / kInvCols), (w + 31) / 32 * 32,
+                kSmem, s, L, ldl, w, T, ldt);
 }
 
 void launch_trsm_lower_unit(const double* L, long long ldl, double* B, long long ldb, int w, int nc,
@@ -298,7 +302,8 @@ void launch_trsm_lower_unit(const double* L, long long ldl, double* B, long long
   configure();
   const int grid = (nc + kTrsmCols - 1) / kTrsmCols;
   dp::note_launch();
-  trsm_lower_unit_kernel<<<grid, kTrsmThreads, kTrsmSmem, s>>>(L, ldl, B, ldb, w, nc, gate);
+  launch_behind(trsm_lower_unit_kernel, dim3(grid), kTrsmThreads, kTrsmSmem, s, L, ldl, B, ldb, w,
+                nc, gate);
 }
 
 void launch_trsm_upper(const double* U, long long ldu, double* B, long long ldb, int w, int nc,

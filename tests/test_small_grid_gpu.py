@@ -66,3 +66,37 @@ def test_block_inverse(built, w):
             for s, e in ((s, min(s + w, n)) for s in range(0, n, w)))
     bound = 2 * n * U * (1 + t) * (np.abs(lower) @ np.abs(upper)).max()
     assert np.abs(a[p][:, q] - lower @ upper).max() <= bound
+
+
+def test_update_behind_others_and_under_capture(built):
+    """A chain of updates, each reading what the one before wrote, is the same bits
+    launched on a stream (each in place before the last has left) and replayed."""
+    import delayed_pivoting as dp
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    n = 96
+    g = torch.Generator().manual_seed(1)
+    a = (torch.randn(n, n, dtype=torch.float64, generator=g) / n).cuda()
+    base = torch.randn(12, n, n, dtype=torch.float64, generator=g).cuda()
+
+    def chain(x, stream):
+        for i in range(1, 12):
+            assert dp.schur_update_device(n, n, n, a, n, x[i - 1], n, x[i], n, stream=stream) == dp.SUCCESS
+
+    direct, replayed = base.clone(), base.clone()
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    chain(direct, s)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(replayed, torch.cuda.current_stream())
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(direct, replayed)
+    want = base.cpu().numpy()
+    for i in range(1, 12):
+        want[i] -= want[i - 1] @ a.cpu().numpy()
+    assert np.abs(direct.cpu().numpy() - want).max() <= 12 * (n + 2) * U * np.abs(want).max() * n
