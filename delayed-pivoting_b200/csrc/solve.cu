@@ -298,10 +298,46 @@ int launch_residual(const double* A, int lda, int n, const double* B, int ldb, c
   return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
 }
 
+// The same norms of a residual that the update kernel left in R (a CTA a column).
+__global__ void __launch_bounds__(256)
+column_norms_kernel(int n, const double* __restrict__ B, long long ldb, const double* __restrict__ X,
+                    long long ldx, const double* __restrict__ R, long long ldr, int nrhs,
+                    double* norms) {
+  __shared__ double part[3][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x;
+  double m[3] = {0.0, 0.0, 0.0};
+  for (int i = threadIdx.x; i < n; i += 256) {
+    m[0] = fmax(m[0], finite_or_inf(R[i + c * ldr]));
+    m[1] = fmax(m[1], finite_or_inf(X[i + c * ldx]));
+    m[2] = fmax(m[2], finite_or_inf(B[i + c * ldb]));
+  }
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m[t] = fmax(m[t], __shfl_down_sync(~0u, m[t], off));
+    if (lane == 0) part[t][warp] = m[t];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = part[threadIdx.x][0];
+    for (int w = 1; w < 8; ++w) v = fmax(v, part[threadIdx.x][w]);
+    norms[(size_t)threadIdx.x * nrhs + c] = v;
+  }
+}
+
 // R = B - A X and berr = max over columns of ||R_c|| / (normA ||X_c|| +
 // ||B_c||), all infinity norms.  `head` (device, solve_head_bytes(nrhs)):
 // the solve's status word, then the norms; a timed-out solve is reported.
 size_t solve_head_bytes(int nrhs) { return 16 + sizeof(double) * 3 * (size_t)nrhs; }
+
+// From 16 right-hand sides on the residual is a contraction for the FP64 tensor
+// cores, once it is large enough to pay for a copy and a launch more.  A solve in
+// ms, residual kernel / update: 16 right-hand sides n = 4096 0.47 / 0.49, 8192
+// 1.26 / 1.07; 32: 2311 0.30 / 0.31, 4096 0.65 / 0.54, 16384 6.6 / 3.6; 64: 2311
+// 0.42 / 0.35, 16384 11.4 / 6.2.
+bool residual_by_update(int n, int nrhs) {
+  return nrhs >= 16 && (long long)n * nrhs >= 1 << 17;
+}
 
 int backward_error(const double* A, int lda, int n, const double* B, int ldb, const double* X,
                    int ldx, int nrhs, double* R, char* head, double normA, double& berr,
@@ -312,14 +348,22 @@ int backward_error(const double* A, int lda, int n, const double* B, int ldb, co
   // no more than eight while the CTAs would not fill the device: n = 2311 with
   // 32 has 73 row blocks
   const int blocks = (n + 31) / 32, sms = sm_count();
-  int nc = nrhs <= 1 ? 1 : nrhs <= 4 ? 4 : nrhs <= 8 ? 8 : nrhs <= 16 ? 16 : 32;
+  int nc = nrhs <= 1 ? 1 : nrhs <= 4 ? 4 : nrhs <= 8 ? 8 : 16;
   while (nc > 8 && (long long)blocks * ((nrhs + nc - 1) / nc) < sms) nc /= 2;
   auto launch = nc == 1    ? launch_residual<1>
                 : nc == 4  ? launch_residual<4>
                 : nc == 8  ? launch_residual<8>
-                : nc == 16 ? launch_residual<16>
-                           : launch_residual<32>;
-  if (int rc = launch(A, lda, n, B, ldb, X, ldx, nrhs, R, norms, st)) return rc;
+                           : launch_residual<16>;
+  if (residual_by_update(n, nrhs)) {
+    note_launch();
+    copy_kernel<<<grid_of((long long)n * nrhs), 256, 0, st>>>(B, ldb, R, n, n, nrhs);
+    launch_gemm_minus(n, nrhs, n, A, lda, X, ldx, R, n, st);
+    note_launch();
+    column_norms_kernel<<<nrhs, 256, 0, st>>>(n, B, ldb, X, ldx, R, n, nrhs, norms);
+    if (cudaGetLastError() != cudaSuccess) return kCudaFailure;
+  } else if (int rc = launch(A, lda, n, B, ldb, X, ldx, nrhs, R, norms, st)) {
+    return rc;
+  }
   std::vector<double> own;
   const size_t bytes = solve_head_bytes(nrhs);
   const double* h = static_cast<const double*>(pinned_stage(bytes));
