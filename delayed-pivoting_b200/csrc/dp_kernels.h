@@ -118,17 +118,18 @@ void launch_gemm_minus(int M, int N, int K, const double* A, long long lda, cons
 void launch_gemm_minus_if(int M, int N, int K, const double* A, long long lda, const double* B,
                           long long ldb, double* C, long long ldc, cudaStream_t s, const int* run);
 
-// C(M x N) -= A(M x K) * B(K x N) to FP64 accuracy on the integer tensor cores
-// (gemm_i8.cu), K <= i8_max_k().  launch_i8_split_a takes A's digits (M <= m
-// rows) and the balance of the K terms from the first `cols` columns of B; any
-// number of updates with that A then follow on the same stream, each over up to
-// n columns.  An operand outside the scheme makes the FP64 kernel do the
-// update.  Return status codes.
+// C(M x N) -= A(M x K) * B(K x N) on the integer tensor cores (gemm_i8.cu), K <=
+// i8_max_k(), where the operands show that no element is further off than its
+// FP64 sum, and else by the FP64 kernel.  launch_i8_split_a takes A's digits (M <=
+// m rows) and the balance of the K terms from the first of the `cols` columns of
+// B; any number of updates with that A then follow on the same stream, each over
+// up to n columns.  Once an update has gone to the FP64 kernel, so do those
+// after it.  Return status codes.
 int i8_max_k();
 size_t i8_bytes(long long m, long long n);  // of the memory behind an I8Update
 struct I8Update {
   void *a_digits = nullptr, *b_digits = nullptr;
-  int *bad = nullptr, *ks = nullptr;
+  int *bad = nullptr, *least = nullptr, *ks = nullptr;
 };
 I8Update i8_update(void* mem, long long m, long long n);
 int launch_i8_split_a(const I8Update& u, int M, int K, const double* A, long long lda,

@@ -15,6 +15,7 @@
 // registers so shared-memory latency hides behind the previous k-step's MMAs.  The C tile is prefetched into L2 when
 // the CTA starts so the read-modify-write of the epilogue hits L2.
 // Accumulation is C - sum_k(a*b), the sum formed in FP64 by the tensor core.
+#include <algorithm>
 #include <atomic>
 
 #include "delayed_pivoting_b200.h"
@@ -214,15 +215,16 @@ dgemm_minus_kernel(int M, int N, int K, const double* __restrict__ A, long long 
   tile_minus<C>(m0, n0, M, N, K, A, lda, B, ldb, Cm, ldc, lower);
 }
 
-// The whole update by a grid of any size, and only when *run < 0.
+// The update when *run < 0 only, `per` tiles a CTA.
 template <class C>
 __global__ void __launch_bounds__(C::THREADS, C::MINB)
 dgemm_minus_if_kernel(int M, int N, int K, const double* __restrict__ A, long long lda,
                       const double* __restrict__ B, long long ldb, double* Cm, long long ldc,
-                      const int* run) {
+                      const int* run, int per) {
   if (*run >= 0) return;
   const long long tm = (M + C::BM - 1) / C::BM, tiles = tm * ((N + C::BN - 1) / C::BN);
-  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+  const long long first = (long long)blockIdx.x * per, last = min(tiles, first + per);
+  for (long long t = first; t < last; ++t) {
     tile_minus<C>(t % tm * C::BM, t / tm * C::BN, M, N, K, A, lda, B, ldb, Cm, ldc, false);
     __syncthreads();  // the stages are free
   }
@@ -319,16 +321,23 @@ void launch_gemm_minus(int M, int N, int K, const double* A, long long lda, cons
     gemm::launch<gemm::Small4>(M, N, K, A, lda, B, ldb, C, ldc, s, gate);
 }
 
-// C -= A * B when *run < 0 (read when the kernel starts), nothing otherwise:
-// few CTAs over all tiles, since this launch nearly always has nothing to do.
+// C -= A * B when *run < 0 (read when the kernel starts), nothing otherwise.  The
+// launch mostly has nothing to do, so a CTA takes several tiles; few, since a CTA
+// that stays long keeps the panels of the next block off its SM.  LU of n = 16384,
+// ms, 1 / 8 / 64 tiles a CTA: none of the updates its own 93.5 / 92.7 / 93.0, all
+// of them (entries exp(2 N(0, 1))) 126.8 / 133.8 / 146.8 (the FP64 update alone in
+// its place took 137.8).
 void launch_gemm_minus_if(int M, int N, int K, const double* A, long long lda, const double* B,
                           long long ldb, double* C, long long ldc, cudaStream_t s, const int* run) {
   if (M <= 0 || N <= 0 || K <= 0) return;
   using Tile = gemm::Small4;
+  constexpr int kPer = 8;
   ensure_smem((const void*)gemm::dgemm_minus_if_kernel<Tile>, Tile::SMEM);
+  const long long tiles = ((M + Tile::BM - 1LL) / Tile::BM) * ((N + Tile::BN - 1LL) / Tile::BN);
+  const int per = (int)std::max(1LL, std::min<long long>(kPer, tiles / (Tile::MINB * sm_count())));
   note_launch();
-  gemm::dgemm_minus_if_kernel<Tile><<<4 * sm_count(), Tile::THREADS, Tile::SMEM, s>>>(
-      M, N, K, A, lda, B, ldb, C, ldc, run);
+  gemm::dgemm_minus_if_kernel<Tile><<<(unsigned)((tiles + per - 1) / per), Tile::THREADS,
+                                      Tile::SMEM, s>>>(M, N, K, A, lda, B, ldb, C, ldc, run, per);
 }
 
 // Lower triangle of the symmetric N x N block C -= A(N x K) * B(K x N), the

@@ -12,21 +12,35 @@
 // 2^26), and the 36 products with d <= 7 are added in FP64 with their weights
 // 2^(-8 d), smallest first.
 //
-// Error: the digits are off by at most 2^-64 of their row's (column's) largest
-// entry, and the products left out (d >= 8) sum to about 2^-60 max|a_i.|
-// max|b_.j| over K = 256 terms.  That is far below an FP64 sum's rounding of
-// those terms, and has to be: in an LU the terms are several times larger than
-// their sum, which the elimination's order keeps small on the FP64 path.
-// Measured on L21 U12 of an N(0, 1) matrix (n = 4096, K = 256): FP64 path
-// 2.4e-15, seven digits (28 products, a quarter faster) 8.6e-15.  Integers up
-// to 2^62 times a row's scale, exact zeros and zero columns stay exact.  Each
-// scale puts the largest entry just below 127.5, the whole range of the first
-// digit.
+// Error: with alpha_i and beta_j the largest scaled entries of row i of A and
+// column j of B, the ends of the digits and the products left out (d >= 8) come
+// to about 2^-59 alpha_i beta_j over K = 256 terms, whatever the sizes of the
+// terms themselves.  An FP64 sum errs by some 2^-55 of sum_k |a_ik b_kj|.  So the
+// scheme is the better one where that sum is not far below alpha_i beta_j, and
+// loses every bit where the two maxima stand in different terms: rows of U12 that
+// are large in some columns and small, or zero, in others.  Two steps keep it to
+// the first kind:
+//   balance  the terms are scaled by 2^+-ks[k], the size of row k of U12 in a
+//            sample of columns, each column in units of its own size, so that the
+//            rows' order of magnitude (the pivots') does not count (row_scale_kernel);
+//   proof    the split kernels add up min(1, 16 |a'_ik| / alpha_i) for every row
+//            and min(1, 16 |b'_kj| / beta_j) for every column.  xy >= x + y - 1
+//            holds in [0, 1], so that two sums that exceed K + 32 together show
+//            sum_k |a_ik b_kj| >= 32 / 256 alpha_i beta_j: every element is then
+//            at least as close as its FP64 sum.  Dense operands have margin (N(0, 1)
+//            from n = 2560 to 16384, rows or columns of scales 1e-20 to 1e20:
+//            smallest sums 0.52 K and 0.70 K), and zero rows, columns and terms
+//            cost none.  Where the least of the rows' sums and a column's fall short
+//            the update is the FP64 kernel's.
+// Measured on L21 U12 of an N(0, 1) matrix (n = 4096, K = 256): FP64 path 2.4e-15,
+// seven digits (28 products, a quarter faster) 8.6e-15.  Integers up to 2^62 times
+// a row's scale, exact zeros and zero columns stay exact.  Each scale puts the
+// largest entry just below 127.5, the whole range of the first digit.
 //
-// Operands outside the scheme - a NaN, an infinity, or a row / column whose
-// largest entry is outside 2^+-kMaxExp - set a flag on the device: the kernel
-// then does nothing and the FP64 kernel behind it does the update (its CTAs
-// return at once otherwise).
+// Operands outside the scheme - those without the proof, a NaN, an infinity, or a
+// row / column whose largest entry is outside 2^+-kMaxExp - set a flag on the
+// device: the kernel then does nothing and the FP64 kernel behind it does the
+// update (its CTAs return at once otherwise).
 //
 // Pipeline: split kernels write the digits as the shared-memory images of 128
 // (A) or 64 (B) rows x 32 bytes of K, all eight digits of a piece side by side,
@@ -43,7 +57,7 @@
 // four accumulators, each pass waiting for the reads of the one before) took
 // 583 us for 8192 x 8192 x 256.
 #include <algorithm>
-#include <mutex>
+#include <climits>
 
 #include "dp_device.cuh"
 #include "dp_kernels.h"
@@ -64,6 +78,7 @@ constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kEpiCols = BN / (kEpiWarps / 4);  // 16 columns per epilogue thread
 constexpr unsigned kTmemCols = 512;
 constexpr int kMaxK = 256;
+constexpr int kScaleCols = 64;  // columns of U12 that balance the K terms
 
 // Byte of (row, k) inside a piece's image: 8 rows x 16 bytes contiguous, the
 // two 16-byte halves of K side by side, then the next 8 rows.
@@ -112,40 +127,71 @@ __device__ __forceinline__ void digit_words(const double (&x)[4], double up,
   }
 }
 
-// Balance of the K terms: ks[k] = the exponent of the largest of the first
-// `cols` entries of row k of B.  A's columns are scaled by 2^ks[k] and B's rows
-// by 2^-ks[k] before the digits are taken.  Without it, rows of very different
-// size in the matrix being factored (row k of U small, its multipliers large)
-// put the terms that matter below the digits of the row's largest multiplier.
+// Balance of the K terms: ks[k] = the exponent of the largest of the first `cols`
+// (at most kScaleCols) entries of row k of B, each in units of the largest of its
+// column.  A's columns are scaled by 2^ks[k] and B's rows by 2^-ks[k] before the
+// digits are taken.  Without it, rows of very different size in the matrix being
+// factored (row k of U small, its multipliers large) put the terms that matter
+// below the digits of the row's largest multiplier.  A row without an entry there
+// takes the smallest exponent of the others, which raises no row of A.  Also sets
+// the operands' flag and the least sum of A's rows (split_a_kernel) to their start.
 __global__ void __launch_bounds__(kMaxK) row_scale_kernel(const double* __restrict__ B,
                                                           long long ldb, int K, int cols, int* ks,
-                                                          int* bad) {
+                                                          int* bad, int* least) {
+  __shared__ int top[kScaleCols], low;
   const int k = threadIdx.x;
-  if (k >= K) return;
-  double m = 0.0;
-  for (int c0 = 0; c0 < cols; c0 += 16) {
-    double v[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = c0 + u < cols ? B[idx(k, c0 + u, ldb)] : 0.0;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) m = fmax(m, fabs(v[u]));
+  if (k < kScaleCols) top[k] = 0;
+  if (k == 0) {
+    low = INT_MAX;
+    *bad = 0;
+    *least = INT_MAX;
   }
-  int e;
-  const bool ok = scale_exponent(m, e);
-  ks[k] = ok ? e : 0;
-  if (!ok) *bad = -1;
+  __syncthreads();
+  int mine = INT_MIN;
+  for (int pass = 0; pass < 2; ++pass) {  // the columns' sizes, then the rows'
+    for (int c0 = 0; c0 < cols; c0 += 16) {
+      int e[16];  // biased exponents, 0 for zero
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        e[u] = k < K && c0 + u < cols ? (__double2hiint(B[idx(k, c0 + u, ldb)]) >> 20) & 0x7ff : 0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        if (pass == 0) {
+          const int m = __reduce_max_sync(~0u, e[u]);
+          if ((k & 31) == 0 && m > 0) atomicMax(&top[c0 + u], m);
+        } else if (e[u] > 0) {
+          mine = max(mine, e[u] - top[c0 + u]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  const int least_here = __reduce_min_sync(~0u, mine == INT_MIN ? INT_MAX : mine);
+  if ((k & 31) == 0) atomicMin(&low, least_here);
+  __syncthreads();
+  if (mine == INT_MIN) mine = low == INT_MAX ? 0 : low;
+  if (k < K) ks[k] = max(mine, -kMaxExp);
+}
+
+// Sums of min(1, 16 |x| / largest) are kept in units of 1 / kShare.
+constexpr int kShare = 16, kProof = 32;
+__device__ __forceinline__ float share_of(double x, double per_max) {
+  return fminf(1.0f, (float)(fabs(x) * per_max));
 }
 
 // A (M x K, column-major) -> digit images [row tile][piece][digit], scales ra[m]
-// = 2^e.  32 rows a CTA; the columns arrive a warp a column (coalesced), warp w
-// then packs piece w: a lane its row's 32 columns.
+// = 2^e, the least of the rows' sums in *least (rows of zeros apart).  32 rows a
+// CTA; the columns arrive a warp a column (coalesced), warp w then packs piece w: a
+// lane its row's 32 columns.
 __global__ void __launch_bounds__(256) split_a_kernel(const double* __restrict__ A, long long lda,
                                                       int M, int K, int pieces,
                                                       const int* __restrict__ ks,
                                                       unsigned char* __restrict__ out,
-                                                      double* __restrict__ ra, int* bad) {
+                                                      double* __restrict__ ra, int* bad,
+                                                      int* least) {
   extern __shared__ double tile[];  // [32][kMaxK + 1]
   __shared__ double mx[8][32];
+  __shared__ float part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * 32 + lane;
   double m = 0.0;
@@ -162,9 +208,21 @@ __global__ void __launch_bounds__(256) split_a_kernel(const double* __restrict__
   for (int w = 0; w < 8; ++w) m = fmax(m, mx[w][lane]);
   int e;
   const bool ok = scale_exponent(m, e);
-  if (warp == 0 && row < M) {
-    ra[row] = ok ? pow2(e) : 0.0;
-    if (!ok) *bad = -1;
+  const bool counts = ok && m > 0.0;
+  const double per_max = counts ? 16.0 / m : 0.0;
+  float sum = 0.0f;
+  for (int k = warp; k < K; k += 8) sum += share_of(tile[lane * (kMaxK + 1) + k], per_max);
+  part[warp][lane] = sum;
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) sum += part[w][lane];
+    const int own = __reduce_min_sync(~0u, row < M && counts ? (int)(kShare * sum) : INT_MAX);
+    if (lane == 0) atomicMin(least, own);
+    if (row < M) {
+      ra[row] = ok ? pow2(e) : 0.0;
+      if (!ok) *bad = -1;
+    }
   }
   if (row >= M || warp >= pieces || !ok) return;
   const double up = pow2(63 - e);
@@ -189,16 +247,19 @@ __global__ void __launch_bounds__(256) split_a_kernel(const double* __restrict__
 }
 
 // B (K x N, column-major) -> digit images [column tile][piece][digit], scales
-// cb[n] = 2^(e - 70).  A warp per column, a lane packs 8 consecutive rows.
+// cb[n] = 2^(e - 70), and the proof for each column: its sum beside the least of
+// A's rows.  A warp per column, a lane packs 8 consecutive rows.
 __global__ void __launch_bounds__(256) split_b_kernel(const double* __restrict__ B, long long ldb,
                                                       int K, int N, int pieces,
                                                       const int* __restrict__ ks,
                                                       unsigned char* __restrict__ out,
-                                                      double* __restrict__ cb, int* bad) {
+                                                      double* __restrict__ cb, int* bad,
+                                                      const int* __restrict__ least) {
   __shared__ double buf[8][kMaxK + kMaxK / 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = blockIdx.x * 8 + warp;
   if (n >= N) return;
+  if (__shfl_sync(~0u, *bad, 0) < 0) return;  // (one answer a warp; *bad stays)
   double m = 0.0;
   bool nan = false;
   for (int k = lane; k < kMaxK; k += 32) {
@@ -213,9 +274,18 @@ __global__ void __launch_bounds__(256) split_b_kernel(const double* __restrict__
   __syncwarp();
   int e;
   const bool ok = scale_exponent(m, e);
+  const double per_max = ok && m > 0.0 ? 16.0 / m : 0.0;
+  float sum = 0.0f;
+#pragma unroll
+  for (int k = lane; k < kMaxK; k += 32) sum += share_of(buf[warp][k + (k >> 3)], per_max);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(~0u, sum, off);
   if (lane == 0) {
     cb[n] = ok ? pow2(e - 70) : 0.0;
-    if (!ok) *bad = -1;
+    // (*least is INT_MAX when every row of A is zero)
+    const bool proven = m == 0.0 || (int)(kShare * sum) + min(*least, kShare * K) >=
+                                        kShare * (K + kProof);
+    if (!ok || !proven) *bad = -1;
   }
   if (!ok || 8 * lane >= pieces * BK) return;
   const double up = pow2(63 - e);
@@ -445,7 +515,7 @@ double* scales_of(void* digits, long long rows) {
 }  // namespace
 
 size_t i8_bytes(long long m, long long n) {
-  return i8_digits_bytes(m) + i8_digits_bytes(n) + i8::al(sizeof(int) * (i8::kMaxK + 1));
+  return i8_digits_bytes(m) + i8_digits_bytes(n) + i8::al(sizeof(int) * (i8::kMaxK + 2));
 }
 
 I8Update i8_update(void* mem, long long m, long long n) {
@@ -454,21 +524,22 @@ I8Update i8_update(void* mem, long long m, long long n) {
   u.a_digits = p;
   u.b_digits = p + i8_digits_bytes(m);
   u.bad = reinterpret_cast<int*>(p + i8_digits_bytes(m) + i8_digits_bytes(n));
-  u.ks = u.bad + 1;
+  u.least = u.bad + 1;
+  u.ks = u.bad + 2;
   return u;
 }
 
 int launch_i8_split_a(const I8Update& u, int M, int K, const double* A, long long lda,
                       const double* B, long long ldb, int cols, cudaStream_t s) {
   const size_t smem = sizeof(double) * 32 * (i8::kMaxK + 1);
-  if (M <= 0 || K <= 0 || K > i8::kMaxK || !ensure_smem((const void*)i8::split_a_kernel, smem) ||
-      cudaMemsetAsync(u.bad, 0, sizeof(int), s) != cudaSuccess)
+  if (M <= 0 || K <= 0 || K > i8::kMaxK || !ensure_smem((const void*)i8::split_a_kernel, smem))
     return kCudaFailure;
   note_launch(2);
-  i8::row_scale_kernel<<<1, i8::kMaxK, 0, s>>>(B, ldb, K, cols, u.ks, u.bad);
+  i8::row_scale_kernel<<<1, i8::kMaxK, 0, s>>>(B, ldb, K, std::min(cols, i8::kScaleCols), u.ks,
+                                               u.bad, u.least);
   i8::split_a_kernel<<<(M + 31) / 32, 256, smem, s>>>(
       A, lda, M, K, (K + i8::BK - 1) / i8::BK, u.ks, static_cast<unsigned char*>(u.a_digits),
-      scales_of(u.a_digits, M), u.bad);
+      scales_of(u.a_digits, M), u.bad, u.least);
   return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
 }
 
@@ -482,7 +553,7 @@ int launch_gemm_minus_i8(const I8Update& u, int M, int N, int K, const double* A
   note_launch(2);
   split_b_kernel<<<(N + 7) / 8, 256, 0, s>>>(B, ldb, K, N, pieces, u.ks,
                                              static_cast<unsigned char*>(u.b_digits),
-                                             scales_of(u.b_digits, N), u.bad);
+                                             scales_of(u.b_digits, N), u.bad, u.least);
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   // two tiles a CTA: more of them keep the tensor path busier (8192 x 8192 alone:
   // 4 a CTA 666 us, all of an SM's 598), fewer give the SMs back sooner to the

@@ -405,7 +405,6 @@ struct I8Block {
   I8Update u;
   bool ready = false;
 };
-constexpr int kI8ScaleCols = 64;  // columns of U12 that balance the W terms
 
 // Where it is used: below about 2000 x 2000 the splits and the tensor path's
 // start eat the gain (K = 256, FP64 path / this, us: 1024 x 1024 32 / 37,
@@ -449,7 +448,7 @@ int update_columns(double* a, long long lda, int m, int s0, int W, int r_gemm, i
     const double *A = a + idx(r_gemm, s0, lda), *U = a + idx(s0, c0, lda);
     int e = kOk, launches = 3;
     if (!i8->ready) {
-      e = launch_i8_split_a(i8->u, M, W, A, lda, U, lda, std::min(kI8ScaleCols, nc), st);
+      e = launch_i8_split_a(i8->u, M, W, A, lda, U, lda, nc, st);
       i8->ready = true;
       launches += 2;
     }
@@ -827,11 +826,18 @@ int factorize(int m, int n, double* a, long long lda, const Options& o, Workspac
       if (E < n) block_inverse(B, E - B, 0, inv1, inv2);
       const int NE = std::min(pivots, E + NB);
       I8Block* i8 = integer_update(E, NE, E - B, i8blk);
-      if (i8)  // the next block's columns first, as with look-ahead
+      // the integer update in the parts that look-ahead makes of it: a part may
+      // go to the FP64 kernel, and then those after it
+      const int NNE = i8 ? std::min(pivots, NE + NB) : NE;
+      if (i8) {
         if (int err = update_columns(a, lda, m, B, E - B, E, E, NE, st, rec, nullptr,
                                      &ws.state->status, terms, nullptr, &inv2))
           return err;
-      if (int err = update_columns(a, lda, m, B, E - B, E, i8 ? NE : E, n, st, rec, mixed_ws,
+        if (int err = update_columns(a, lda, m, B, E - B, E, NE, NNE, st, rec, mixed_ws,
+                                     &ws.state->status, terms, nullptr, &inv2, false, i8))
+          return err;
+      }
+      if (int err = update_columns(a, lda, m, B, E - B, E, i8 ? NNE : E, n, st, rec, mixed_ws,
                                    &ws.state->status, terms, nullptr, &inv2, false, i8))
         return err;
       DP_CHECK_CUDA(cudaGetLastError());
