@@ -78,16 +78,14 @@ struct Job {
   dp_request r{};
   double t_submit = 0, t_admit = 0;
   size_t scratch = 0, factor = 0;    // charged bytes
+  bool alone = false;                // not coalesced: charged for a solve by itself
   std::shared_ptr<Resident> res;     // follow-ups
 };
 
-// X, R and the two buffers of one solve, its columns in a coalesced solve.
-size_t scratch_bytes(int n, int nrhs) { return 5 * sizeof(double) * (size_t)n * nrhs + 4096; }
-
-// The smallest scratch a budget must hold beside the factor for a request to
-// be accepted; one between the two is charged all that the budget has left.
-size_t least_scratch_bytes(int n, int nrhs) {
-  return 4 * sizeof(double) * (size_t)n * nrhs + 4096;
+// Device memory of a request's solve: X, R and the two buffers of one solve, and
+// its columns where it is coalesced with others.
+size_t scratch_bytes(int n, int nrhs, bool alone) {
+  return (alone ? 4 : 5) * sizeof(double) * (size_t)n * nrhs + 4096;
 }
 
 size_t small_factor_bytes(int n) {
@@ -169,6 +167,11 @@ struct dp_server {
         }
         j.res = rit->second;
       }
+      // room for its columns in a coalesced solve where there is some (without
+      // this choice a follow-up whose five vectors do not fit beside the factor
+      // would wait for ever, though a solve by itself fits)
+      j.alone = used + scratch_bytes(j.r.n, j.r.nrhs, false) + j.factor > budget;
+      j.scratch = scratch_bytes(j.r.n, j.r.nrhs, j.alone);
       const size_t need = j.scratch + j.factor;
       if (used + need > budget) {
         ++it;
@@ -220,11 +223,12 @@ void dp_server::drop_resident_locked(const std::shared_ptr<Resident>& r, cudaStr
 
 // Moves the admitted follow-up solves of factorisation `factor_id` out of
 // the large queue into `batch` while the right-hand sides fit one solve
-// (at most dp::serve::kMaxRhs columns in all).
+// (at most dp::serve::kMaxRhs columns in all), those charged for it.
 void dp_server::take_followups_locked(unsigned long long factor_id, int& rhs,
                                       std::vector<Job>& batch) {
   for (auto it = large_q.begin(); it != large_q.end();) {
-    if (it->r.factor_id == factor_id && rhs + it->r.nrhs <= dp::serve::kMaxRhs) {
+    if (it->r.factor_id == factor_id && !it->alone &&
+        rhs + it->r.nrhs <= dp::serve::kMaxRhs) {
       rhs += it->r.nrhs;
       batch.push_back(*it);
       ++running;
@@ -313,7 +317,8 @@ void dp_server::large_worker() {
       large_q.pop_front();
       ++running;
       rhs = batch[0].r.nrhs;
-      if (batch[0].r.factor_id != 0) take_followups_locked(batch[0].r.factor_id, rhs, batch);
+      if (batch[0].r.factor_id != 0 && !batch[0].alone)
+        take_followups_locked(batch[0].r.factor_id, rhs, batch);
     }
     std::vector<dp_request_result> out(batch.size());
     for (auto& r : out) {
@@ -348,7 +353,7 @@ void dp_server::large_worker() {
         std::lock_guard<std::mutex> lk(m);
         residents[keep->id] = keep;
         schedule_locked();
-        take_followups_locked(keep->id, rhs, batch);
+        if (!batch[0].alone) take_followups_locked(keep->id, rhs, batch);
         out.resize(batch.size());
         for (size_t i = 1; i < out.size(); ++i) {
           out[i].path = 1;
@@ -798,11 +803,10 @@ int dp_server_submit(dp_server* s, const dp_request* q) {
   Job j;
   j.r = r;
   j.t_submit = clock_s();
-  j.scratch = scratch_bytes(r.n, r.nrhs);
+  j.scratch = scratch_bytes(r.n, r.nrhs, true);  // the least; schedule_locked() decides
   if (r.factor_id == 0)
     j.factor = s->is_small(r.n) ? small_factor_bytes(r.n) : large_factor_bytes(r.n);
-  if (least_scratch_bytes(r.n, r.nrhs) + j.factor > s->budget) return DP_INVALID_ARGUMENT;
-  j.scratch = std::min(j.scratch, s->budget - j.factor);
+  if (j.scratch + j.factor > s->budget) return DP_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lk(s->m);
   if (s->stop) return DP_INVALID_ARGUMENT;
   if (r.factor_id == 0) {
