@@ -35,7 +35,8 @@
 //              argmax (smaller column, then smaller row on ties), full-row and
 //              full-column swaps, restart the panel at k with the pivot placed
 // The panel width is chosen per size bucket (dp_batch_options.nb_bucket);
-// dp_batch_autotune fills that table by timing the candidates.
+// dp_batch_autotune fills that table by timing the candidates.  One above the
+// window runs as the window.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -57,6 +58,7 @@ namespace batch {
 
 constexpr int kMaxN = DP_BATCH_MAX_N;
 constexpr int kMaxNb = DP_BATCH_MAX_NB;   // panel width limit
+constexpr int kWindow = 16;               // panel columns a matrix's CTA holds; wider panels run as this
 constexpr int kSb = 8;                    // sub-panel width inside the window
 constexpr int kMaxWarps = 16;
 constexpr int kLeftMoves = 2 * kMaxN;     // row moves kept for the columns on the left,
@@ -977,10 +979,10 @@ size_t dynamic_smem(int max_n) {
 // 20.6, up to 256: 5.3, up to 128: 2.0), 256 threads of two rows for the
 // largest class (18.9; with two CTAs per SM 21.5), tiles of 16 x 32 with the
 // next one's loads in flight (19.1).
-using Geo3 = Geo<512, 1, 16, 256, 4, 1>;
-using Geo2 = Geo<256, 1, 16, 128, 2, 2>;
-using Geo1 = Geo<128, 1, 16, 128, 2, 4>;
-using Geo0 = Geo<64, 1, 16, 64, 1, 7>;
+using Geo3 = Geo<512, 1, kWindow, 256, 4, 1>;
+using Geo2 = Geo<256, 1, kWindow, 128, 2, 2>;
+using Geo1 = Geo<128, 1, kWindow, 128, 2, 4>;
+using Geo0 = Geo<64, 1, kWindow, 64, 1, 7>;
 
 // Panels of the blocked LU: a row per thread (STAGE and the warp grid unused).
 template <int T>
@@ -1178,8 +1180,7 @@ void dp_batch_options_init(dp_batch_options* o) {
   std::memset(o, 0, sizeof(*o));
   o->threshold = 0.0;
   o->precision = DP_PRECISION_FP64;
-  const int defaults[DP_BATCH_BUCKETS] = {16, 16, 32, 32};
-  for (int i = 0; i < DP_BATCH_BUCKETS; ++i) o->nb_bucket[i] = defaults[i];
+  for (int& nb : o->nb_bucket) nb = dp::batch::kWindow;
 }
 
 int dp_batch_create(dp_batch** out, int count, const int* n, const long long* offsets,
@@ -1354,7 +1355,7 @@ int dp_batch_autotune(dp_batch_options* opt, int samples, unsigned long long see
   dp_batch_options base = *opt;
   if (!valid_batch_options(&base)) return DP_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
-  static const int kCand[] = {8, 16, 24, 32};
+  static const int kCand[] = {8, dp::batch::kWindow};
   int rc = DP_SUCCESS;
   for (int bk = 0; bk < DP_BATCH_BUCKETS && rc == DP_SUCCESS; ++bk) {
     const int lo = std::max(kBucketLo[bk], 16), hi = kBucketHi[bk];

@@ -226,7 +226,8 @@ typedef struct dp_batch_options {
                                       decisions in FP64; factors for FP64 refinement,
                                       records may differ where a decision is within the
                                       update's rounding */
-  int nb_bucket[DP_BATCH_BUCKETS]; /* panel width per order bucket, 1..DP_BATCH_MAX_NB */
+  int nb_bucket[DP_BATCH_BUCKETS]; /* panel width per order bucket, 1..DP_BATCH_MAX_NB (the
+                                      kernels hold 16 columns: wider runs as 16); default 16 */
   int reserved[2];
 } dp_batch_options;
 
