@@ -102,11 +102,9 @@ void launch_lower_inverse(const double* L, long long ldl, int w, double* T, long
 // dst <- src for a rows x cols column-major block (device memory).
 void launch_copy_block(const double* src, long long lds, double* dst, long long ldd, int rows,
                        int cols, cudaStream_t s);
-// Same with separate operands; and B <- U^{-1} B for upper U with diagonal.
+// Same with separate operands.
 void launch_trsm_lower_unit(const double* L, long long ldl, double* B, long long ldb, int w, int nc,
                             cudaStream_t s, const int* gate = nullptr);
-void launch_trsm_upper(const double* U, long long ldu, double* B, long long ldb, int w, int nc,
-                       cudaStream_t s);
 
 // C(M x N) -= A(M x K) * B(K x N); all three inside the same column-major
 // matrix (or any column-major operands).  `gate` as for the TRSM.
