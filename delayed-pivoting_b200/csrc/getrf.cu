@@ -1053,19 +1053,24 @@ int getrf_device(int m, int n, double* d_a, int lda, int* ipiv, int* jpiv, int* 
     ip.copy2_cols = n;
   }
   // the first block's update is the largest
-  const size_t i8_mem = !mixed_terms(o.precision) && use_i8(m - (long long)NB, n - 2LL * NB, NB)
-                            ? i8_bytes(m, n)
-                            : 0;
-  const size_t bytes = layout_workspace(ws, nullptr, pivots, di.sms, w_max, mixed_bytes,
-                                        defer_cap, mixed1_bytes, ip, i8_mem);
+  size_t i8_mem = !mixed_terms(o.precision) && use_i8(m - (long long)NB, n - 2LL * NB, NB)
+                      ? i8_bytes(m, n)
+                      : 0;
+  auto layout = [&](char* at) {
+    return layout_workspace(ws, at, pivots, di.sms, w_max, mixed_bytes, defer_cap, mixed1_bytes,
+                            ip, i8_mem);
+  };
   char* base = nullptr;
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&base), bytes, st) != cudaSuccess) {
+  while (dp::workspace_alloc(reinterpret_cast<void**>(&base), layout(nullptr), st) !=
+         cudaSuccess) {
     cudaGetLastError();
-    *info = -1;
-    return kAllocationFailed;
+    if (i8_mem == 0) {
+      *info = -1;
+      return kAllocationFailed;
+    }
+    i8_mem = 0;  // no room for the digits: every update by the FP64 kernel
   }
-  layout_workspace(ws, base, pivots, di.sms, w_max, mixed_bytes, defer_cap, mixed1_bytes, ip,
-                   i8_mem);
+  layout(base);
   int status = kOk;
   // the scratch regions (at the end) are fully written before use; clear the rest
   const size_t clear = (size_t)(ws.scratch - base);
