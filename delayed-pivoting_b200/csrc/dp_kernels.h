@@ -189,19 +189,21 @@ void launch_identity_records(int* ipiv, int* jpiv, int count, cudaStream_t s);
 
 // ---- triangular solves with many right-hand sides (trisolve.cu) ----------
 
-// X <- Q U^{-1} L^{-1} P B (n x nrhs) in one launch per 64 right-hand sides:
+// X <- Q U^{-1} L^{-1} P B (n x nrhs) in one launch per `pass` right-hand sides
+// (at most lu_solve_pass(nrhs), the fastest; no result bit depends on it):
 // row / col are the composite orders (B row row[i] is eliminated i-th, unknown
 // col[i] takes the i-th value), X may be B.  `inv` holds the inverses of the
 // 64 x 64 diagonal blocks of L and U (launch_diag_inverse,
 // tri_inverse_doubles(n) doubles, 16-byte aligned), `work`
-// lu_solve_work_bytes(n, nrhs) bytes; a bounded wait that runs out sets
+// lu_solve_work_bytes(n, pass) bytes; a bounded wait that runs out sets
 // *status = kDeviceTimeout.
 size_t tri_inverse_doubles(int n);
 int launch_diag_inverse(const double* lu, long long ldlu, int n, double* inv, cudaStream_t st);
-size_t lu_solve_work_bytes(int n, int nrhs);
+int lu_solve_pass(int nrhs);
+size_t lu_solve_work_bytes(int n, int pass);
 int launch_lu_solve(const double* lu, long long ldlu, int n, const double* inv, const int* row,
                     const int* col, const double* B, long long ldb, double* X, long long ldx,
-                    int nrhs, void* work, int* status, cudaStream_t st);
+                    int nrhs, void* work, int pass, int* status, cudaStream_t st);
 
 // ---- resident factorisations (solve.cu) ----------------------------------
 

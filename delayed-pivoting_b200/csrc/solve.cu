@@ -162,6 +162,22 @@ int grid_of(long long work) {
 
 }  // namespace
 
+namespace {
+
+// `fixed` bytes and, behind them, the buffers of a solve: for passes as wide as
+// launch_lu_solve makes them, or narrower ones (*pass) where memory is short.
+int solve_alloc(char** mem, size_t fixed, int n, int nrhs, int* pass, cudaStream_t st) {
+  for (*pass = lu_solve_pass(nrhs);; *pass = *pass > 8 ? 8 : 1) {
+    if (dp::workspace_alloc(reinterpret_cast<void**>(mem), fixed + lu_solve_work_bytes(n, *pass),
+                            st) == cudaSuccess)
+      return kOk;
+    cudaGetLastError();
+    if (*pass == 1) return kAllocationFailed;
+  }
+}
+
+}  // namespace
+
 int getrs_device(int n, int nrhs, const double* lu, int ldlu, const int* ipiv, const int* jpiv,
                  double* B, int ldb, cudaStream_t st) {
   if (n < 0 || nrhs < 0 || ldlu < std::max(1, n) || ldb < std::max(1, n)) return kInvalidArgument;
@@ -178,11 +194,8 @@ int getrs_device(int n, int nrhs, const double* lu, int ldlu, const int* ipiv, c
   const size_t b_perm = sizeof(int) * (4 + 2 * (((size_t)n + 1) & ~(size_t)1));
   const size_t b_inv = sizeof(double) * tri_inverse_doubles(n);
   char* mem = nullptr;
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&mem),
-                          b_perm + b_inv + lu_solve_work_bytes(n, nrhs), st) != cudaSuccess) {
-    cudaGetLastError();
-    return kAllocationFailed;
-  }
+  int pass = 0;
+  if (int e = solve_alloc(&mem, b_perm + b_inv, n, nrhs, &pass, st)) return e;
   int* const d_status = reinterpret_cast<int*>(mem);
   int* const d_perm = d_status + 4;
   double* const inv = reinterpret_cast<double*>(mem + b_perm);
@@ -196,7 +209,7 @@ int getrs_device(int n, int nrhs, const double* lu, int ldlu, const int* ipiv, c
   if (status == kOk) status = launch_diag_inverse(lu, ldlu, n, inv, st);
   if (status == kOk)
     status = launch_lu_solve(lu, ldlu, n, inv, d_perm, d_perm + n, B, ldb, B, ldb, nrhs,
-                             mem + b_perm + b_inv, d_status, st);
+                             mem + b_perm + b_inv, pass, d_status, st);
   if (status == kOk &&
       cudaMemcpyAsync(&h, d_status, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     status = kCudaFailure;
@@ -431,11 +444,11 @@ int factorize(Factor& f, const double* A, int lda, int prec, cudaStream_t st) {
 }
 
 // X = A^{-1} B through the factors (X: n x nrhs, leading dimension n; it may
-// be B); `work` as for launch_lu_solve.
-int solve_with(const Factor& f, const double* B, int ldb, double* X, void* work, int nrhs,
+// be B); `work` and `pass` as for launch_lu_solve.
+int solve_with(const Factor& f, const double* B, int ldb, double* X, void* work, int pass, int nrhs,
                int* status, cudaStream_t st) {
   return launch_lu_solve(f.lu, f.n, f.n, f.d_inv, f.d_perm, f.d_perm + f.n, B, ldb, X, f.n, nrhs,
-                         work, status, st);
+                         work, pass, status, st);
 }
 
 // z = A^{-T} c through the factors: A^T = Q U^T L^T P, so with w[k] =
@@ -445,7 +458,7 @@ int solve_with(const Factor& f, const double* B, int ldb, double* X, void* work,
 int solve_transposed(const Factor& f, const double* lut, const double* inv_t, const double* c,
                      double* z, void* work, int* status, cudaStream_t st) {
   return launch_lu_solve(lut, f.n, f.n, inv_t, f.d_perm + f.n, f.d_perm, c, f.n, z, f.n, 1, work,
-                         status, st);
+                         1, status, st);
 }
 
 }  // namespace
@@ -509,7 +522,7 @@ int factor_condest(Factor* f, const double* A, int lda, double* kappa, double* i
       status = kCudaFailure;
   };
   auto forward = [&] {  // y = A^{-1} x (x on the device), copied to hy
-    if (status == kOk) status = solve_with(*f, x, n, y, work, 1, d_status, st);
+    if (status == kOk) status = solve_with(*f, x, n, y, work, 1, 1, d_status, st);
     down(hy, y);
   };
   auto backward = [&] {  // y = A^{-T} x, copied to hy
@@ -715,11 +728,8 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
   const size_t b_head = (solve_head_bytes(nrhs) + 255) / 256 * 256;
   const size_t b_vec = (nr * sizeof(double) + 255) / 256 * 256;
   char* head = nullptr;
-  if (dp::workspace_alloc(reinterpret_cast<void**>(&head),
-                          b_head + 2 * b_vec + lu_solve_work_bytes(n, nrhs), st) != cudaSuccess) {
-    cudaGetLastError();
-    return kAllocationFailed;
-  }
+  int pass = 0;
+  if (int e = solve_alloc(&head, b_head + 2 * b_vec, n, nrhs, &pass, st)) return e;
   double* const X = reinterpret_cast<double*>(head + b_head);
   double* const R = reinterpret_cast<double*>(head + b_head + b_vec);
   void* const work = head + b_head + 2 * b_vec;
@@ -748,7 +758,7 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
         if (it + needed > iters_left + 0.5) return kOk;
       }
       prev = berr;
-      s = solve_with(*f, R, n, R, work, nrhs, d_status, st);
+      s = solve_with(*f, R, n, R, work, pass, nrhs, d_status, st);
       if (s != kOk) return s;
       dp::note_launch();
       axpy_kernel<<<grid_of((long long)nr), 256, 0, st>>>(R, n, X, n, n, nrhs);
@@ -763,7 +773,7 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
   const double fms0 = f->factor_ms - res->factor_ms;
   bool converged = false;
   if (status == kOk) {
-    status = solve_with(*f, B, ldb, X, work, nrhs, d_status, st);
+    status = solve_with(*f, B, ldb, X, work, pass, nrhs, d_status, st);
     if (status == kOk) status = refine(max_iter, converged);
   }
   if (status == kOk && !converged && f->precision != DP_PRECISION_FP64) {
@@ -771,7 +781,7 @@ int factor_solve(Factor* f, const double* A, int lda, double* B, int ldb, int nr
     f->refactored = 1;
     status = factorize(*f, A, lda, DP_PRECISION_FP64, st);
     if (status == kOk && f->info == n) {
-      status = solve_with(*f, B, ldb, X, work, nrhs, d_status, st);
+      status = solve_with(*f, B, ldb, X, work, pass, nrhs, d_status, st);
       if (status == kOk) status = refine(max_iter, converged);
     }
   }

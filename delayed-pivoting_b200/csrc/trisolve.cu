@@ -360,15 +360,15 @@ int launch_diag_inverse(const double* lu, long long ldlu, int n, double* inv, cu
   return cudaGetLastError() == cudaSuccess ? kOk : kCudaFailure;
 }
 
-size_t lu_solve_work_bytes(int n, int nrhs) {
-  return sizeof(double) * 2 * (size_t)n * std::min(nrhs, kTRhs) + 16;
-}
+int lu_solve_pass(int nrhs) { return std::min(nrhs, kTRhs); }
+
+size_t lu_solve_work_bytes(int n, int pass) { return sizeof(double) * 2 * (size_t)n * pass + 16; }
 
 int launch_lu_solve(const double* lu, long long ldlu, int n, const double* inv, const int* row,
                     const int* col, const double* B, long long ldb, double* X, long long ldx,
-                    int nrhs, void* work, int* status, cudaStream_t st) {
+                    int nrhs, void* work, int pass, int* status, cudaStream_t st) {
   if (n <= 0 || nrhs <= 0) return kOk;
-  for (int c0 = 0; c0 < nrhs; c0 += kTRhs) {
+  for (int c0 = 0; c0 < nrhs; c0 += pass) {
     SolveParams p;
     p.lu = lu;
     p.ldlu = ldlu;
@@ -380,7 +380,7 @@ int launch_lu_solve(const double* lu, long long ldlu, int n, const double* inv, 
     p.ldb = ldb;
     p.X = X + (size_t)c0 * ldx;
     p.ldx = ldx;
-    p.nrhs = std::min(kTRhs, nrhs - c0);
+    p.nrhs = std::min(pass, nrhs - c0);
     p.mid = static_cast<double*>(work);
     p.xs = p.mid + (size_t)n * p.nrhs;
     p.counter = reinterpret_cast<int*>(p.xs + (size_t)n * p.nrhs);
