@@ -4,10 +4,11 @@
 //
 // Control flow follows delayed_lu/delayed_dgetrf.cpp:129-251 and its GPU twin
 // delayed_lu_cuda/delayed_dgetrf_cuda.cu:251-368, with the per-pivot work moved
-// to the device: one cooperative panel launch factors a whole panel (all
+// to the device: one panel launch factors a whole panel (all
 // column searches, acceptance tests, swaps, scalings and rank-1 updates stay
-// on the GPU) and the host reads a 64-byte state block once per panel, where
-// the reference made 2 launches + a D2H copy + a stream sync per column.
+// on the GPU) and the host reads a small state block once per outer block and
+// stop (once per panel where a panel is the cooperative grid's), where the
+// reference made 2 launches + a D2H copy + a stream sync per column.
 //   normal panel  : laswp (rows outside the panel) -> TRSM (U12) -> GEMM (A22)
 //   panel stopped at k (no acceptable column pivot, dgetrf.cpp:182-218):
 //                   laswp of the executed steps -> materialize far columns
@@ -398,7 +399,8 @@ struct BlockInv {
   double* copy = nullptr;  // ldt x (columns) doubles
 };
 
-// The rank-W update of a finished block on the integer tensor cores: A's digits
+// The rank-W update of a finished block on the integer tensor cores, or by the
+// FP64 kernel where its operands do not show that this is as accurate: A's digits
 // are taken in the first update_columns call that has it, and serve the calls
 // after it on the same stream (`ready`).
 struct I8Block {

@@ -9,7 +9,9 @@
 // two pools here (workspaces, and factors that outlive a call) keep up to
 // kKeep bytes of unused memory each; more than that goes back at the next
 // synchronisation, and dp_memory_trim or the end of a server gives back the
-// rest.  An allocation that fails is tried once more after a trim.  The pools
+// rest.  Another allocation of the process that runs short gets it without that
+// (2.3 GiB kept, the device otherwise full: a cudaMalloc of 1 GiB more than its
+// free memory succeeded).  An allocation that fails is tried once more after a trim.  The pools
 // are the driver's own, safe for any mix of threads and streams; a block
 // freed on one stream is handed to another only once the free has been
 // reached (no waits between streams are inserted for it).

@@ -5,7 +5,8 @@
 //              factorisations are charged their factor memory plus solve
 //              scratch, follow-up solves their scratch, and a request is
 //              admitted (first come first served, later requests may pass one
-//              that does not fit yet) as soon as the budget has room
+//              that does not fit yet) as soon as the budget has room, if need be
+//              for a solve by itself instead of a coalesced one
 //   small      orders <= small_max_n: one worker thread takes every admitted
 //              small request at once, packs the matrices into one buffer,
 //              factors them in ONE persistent batched launch (batched.cu),

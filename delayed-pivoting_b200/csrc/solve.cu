@@ -4,12 +4,11 @@
 // factorisation P*A*Q = L*U it produces (delayed_lu_cuda/delayed_dgetrf_cuda.hpp:15-21:
 // ipiv / jpiv are swap histories replayed in order, example.cu:61-68) gives
 //   A x = b  <=>  L U y = P b,  x = Q y.
-// getrs: gather b through the row order of ipiv, forward substitution with
-// the unit-lower L and back substitution with U (64-row diagonal blocks on
-// the TRSM kernels, the off-diagonal blocks as FP64 DMMA GEMM updates),
-// scatter y through the column order of jpiv.
-// gesv_ir: factor (mixed precision: BF16x3 tensor-core trailing update, or
-// plain FP64), solve, then refine in FP64: r = b - A x on the FP64 GEMM,
+// getrs: both sweeps and both orders in one launch per 64 right-hand sides
+// (launch_lu_solve), with the inverses of the 64-row diagonal blocks.
+// gesv_ir: factor (mixed precision: BF16x3 / BF16x6 tensor-core trailing update,
+// or plain FP64), solve, then refine in FP64: r = b - A x by residual_kernel, or
+// the FP64 update kernel for many right-hand sides (residual_by_update),
 // backward error max_c ||r_c||_inf / (||A||_inf ||x_c||_inf + ||b_c||_inf),
 // correction through the same factors.  A refinement that stops improving
 // (error not halved) or does not reach the tolerance within max_iter steps

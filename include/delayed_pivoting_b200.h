@@ -420,7 +420,8 @@ int dp_schur_update_mixed_device(int M, int N, int K, const double *A, int lda, 
 int dp_gemm_tile(int tile);
 
 /* CTAs of a solve's launch (both sweeps; solves and refinement; tuning, no
- * result bit depends on it): 0 automatic (min(row blocks, SMs)), g > 0 at
+ * result bit depends on it): 0 automatic (as many as there are blocks of 64
+ * rows times groups of at most 8 right-hand sides, and fit the device), g > 0 at
  * most g, g < 0 one CTA per -g blocks of 64 rows (at most 32).  Returns the
  * previous setting, or -2000 for a setting outside [-1024, 1024]. */
 int dp_tri_solve_grid(int policy);
